@@ -138,9 +138,11 @@ class SpmmOperator:
         self.device_layout = D.build_spmm_device(plan.tiles, self.A, N=self.N, tc_mode=self.cfg.tc_mode)
         self.handle = DeviceSpmmPlan(self.device_layout)
         self._transposed = None
-        # values last loaded with set_values (a device copy, CSR order); None
-        # while the plan still holds the values of A it was built from
-        self._vals = None
+        # values last loaded with set_values (a device copy, CSR order, or
+        # (the copy of the operator this one is the transposed of, its
+        # permutation)); None while the plan still holds the values of A it
+        # was built from
+        self._vals_src = None
         # (weak reference to the tensor, its version, its address) of the
         # values HybridSpMMFunction loaded last
         self._values_key = None
@@ -154,6 +156,14 @@ class SpmmOperator:
         # (bf16 zero-filled A, nonzero rows, nonzero columns) of the dense
         # forward (built on first use)
         self._dense = None
+
+    @property
+    def _vals(self):
+        """The values last loaded, in this operator's CSR order, or None."""
+        if isinstance(self._vals_src, tuple):
+            vals, perm = self._vals_src
+            self._vals_src = vals[perm]
+        return self._vals_src
 
     def _plain_ops(self):
         if self._plain is None:
@@ -306,9 +316,19 @@ class SpmmOperator:
             W, rows, cols = self._dense
             W[rows, cols] = vals.to(torch.bfloat16)
         self.handle.set_values(vals)
-        self._vals = vals.clone()
+        self._vals_src = vals.clone()
         if self._transposed is not None:
-            self._transposed[0].set_values(self._vals[self._transposed[1]])
+            opT, perm_t = self._transposed
+            opT._set_values_forward(self._vals, perm_t)
+
+    def _set_values_forward(self, vals, perm):
+        """set_values(vals[perm]) of a transposed operator, without the
+        permuted copy unless something other than the plan needs it."""
+        if self._plain is not None or self._dense is not None or self._transposed is not None:
+            self.set_values(vals[perm])
+            return
+        self.handle.set_values_forward(vals)
+        self._vals_src = (vals, perm)
 
     @property
     def transposed(self):

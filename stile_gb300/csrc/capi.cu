@@ -60,6 +60,8 @@ struct StileSpmmPlan {
   int n_zero_rows = 0;
   const int* zero_rows = nullptr;
   long n_tc_dv = 0;  // tensor-tile nonzeros of the value-gradient list
+  long n_tc_live = 0;  // live elements of the tensor-tile value images
+  bool ids_set = false;  // set_transpose_ids has run
 };
 
 // default of the tensor tiles' value gradients: the row runs (measured
@@ -310,16 +312,12 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
 
   // packed entries; an entry ends its run when the next one in its group
   // has another row code (or there is none)
-  std::vector<int32_t> e_ent((size_t)n_pos * 4);
+  std::vector<int32_t> e_ent((size_t)n_pos * 2);
   for (size_t g = 0; g + 1 < e_gptr.size(); ++g)
     for (long q = e_gptr[g]; q < e_gptr[g + 1]; ++q) {
-      int32_t vbits;
-      std::memcpy(&vbits, &e_val[q], 4);
-      e_ent[q * 4 + 0] = e_col[q];
-      e_ent[q * 4 + 1] = vbits;
       const int32_t end = (q + 1 == e_gptr[g + 1] || e_rc[q + 1] != e_rc[q]) ? 1 : 0;
-      e_ent[q * 4 + 2] = e_rc[q] * 2 + end;  // row code and run end in one field
-      e_ent[q * 4 + 3] = 0;
+      e_ent[q * 2 + 0] = e_col[q];
+      e_ent[q * 2 + 1] = e_rc[q] * 2 + end;  // row code and run end in one field
     }
   std::sort(zero.begin(), zero.end());
   zero.erase(std::unique(zero.begin(), zero.end()), zero.end());
@@ -384,6 +382,29 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
     ck_item.swap(item2);
     ck_flags.swap(flags2);
     if (pos != h->tc_n_ksteps) return fail(STILE_E_INVALID, "tensor-core chunks do not cover the k-steps");
+  }
+
+  // live elements of the value images (schedule order): a 256-bit mask per
+  // k-step and the ids of its nonzeros, both in image order
+  std::vector<uint8_t> live_mask;
+  std::vector<int32_t> live_ptr, live_id;
+  if (h->tc_nnz_id && h->tc_n_ksteps > 0) {
+    int src_of[256];  // image element -> row-major (row, column)
+    for (int n = 0; n < 16; ++n)
+      for (int k = 0; k < 16; ++k) src_of[(n >> 3) * 128 + (k >> 3) * 64 + (n & 7) * 8 + (k & 7)] = n * 16 + k;
+    live_mask.assign((size_t)h->tc_n_ksteps * 32, 0);
+    live_ptr.reserve((size_t)h->tc_n_ksteps + 1);
+    live_ptr.push_back(0);
+    for (long ks = 0; ks < h->tc_n_ksteps; ++ks) {
+      for (int i = 0; i < 256; ++i) {
+        const int32_t id = s_nnz[(size_t)ks * 256 + src_of[i]];
+        if (id < 0) continue;
+        live_mask[(size_t)ks * 32 + (i >> 3)] |= (uint8_t)(1u << (i & 7));
+        live_id.push_back(id);
+      }
+      if ((long)live_id.size() > INT32_MAX) return fail(STILE_E_INVALID, "too many tensor-tile entries");
+      live_ptr.push_back((int32_t)live_id.size());
+    }
   }
 
   // value-gradient entry list from the tiles (needs the nonzero ids)
@@ -460,6 +481,10 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
   size_t i_ctac = ar.add(cta_chunk.data(), cta_chunk.size() * 4);
   size_t i_egptr = ar.add(e_gptr.data(), e_gptr.size() * 4);
   size_t i_eent = ar.add(e_ent.data(), e_ent.size() * 4);
+  size_t i_eval = ar.add(e_val.data(), e_val.size() * 4);
+  size_t i_lmask = ar.add(live_mask.data(), live_mask.size());
+  size_t i_lptr = ar.add(live_ptr.data(), live_ptr.size() * 4);
+  size_t i_lid = ar.add(live_id.data(), live_id.size() * 4);
   size_t i_enid = ar.add(e_id.data(), e_id.size() * 4);
   size_t i_zero = ar.add(zero.data(), zero.size() * 4);
   size_t i_ckb = ar.add(ck_kbeg.data(), (size_t)nck * 4);
@@ -517,7 +542,12 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
   a.ell_n_groups = (int)e_gptr.size() - 1;
   a.ell_n_pos = n_pos;
   a.ell_group_ptr = (const int*)P(i_egptr);
-  a.ell_entry = (const int4*)P(i_eent);
+  a.ell_entry = (const int2*)P(i_eent);
+  a.ell_val = (const float*)P(i_eval);
+  a.tc_live_mask = (const uint8_t*)P(i_lmask);
+  a.tc_live_ptr = (const int*)P(i_lptr);
+  a.tc_live_id = (const int*)P(i_lid);
+  plan->n_tc_live = (long)live_id.size();
   a.ell_nnz_id = h->ell_nnz_id ? (const int*)P(i_enid) : nullptr;
   a.err_flag = plan->err_flag;
   a.tc_row_scale = fp8 ? (const float*)P(i_rsc) : nullptr;
@@ -581,8 +611,8 @@ static int check_dense(long ld, int N, const void* ptr, const char* name) {
   return STILE_OK;
 }
 
-// value sets of a batched run: ELL records, then tensor-tile images, per head
-static size_t values_ell_bytes(const StileSpmmPlan* plan) { return (size_t)plan->ell_n_slots * 16; }
+// value sets of a batched run: ELL values, then tensor-tile images, per head
+static size_t values_ell_bytes(const StileSpmmPlan* plan) { return (size_t)plan->ell_n_slots * 4; }
 static size_t values_tc_bytes(const StileSpmmPlan* plan) {
   const size_t kb = plan->args.tc_mode == STILE_TC_SPLIT_BF16 ? 1024 : 512;
   return (size_t)plan->args.tc_n_ksteps * kb;
@@ -663,7 +693,7 @@ static int spmm_run(const StileSpmmPlan* plan, const void* B, bool b_bf16, int64
     a.b_head_stride = hd.b_stride;
     a.c_head_stride = hd.c_stride;
     const uint8_t* pk = static_cast<const uint8_t*>(hd.packed);
-    a.ell_entry = reinterpret_cast<const int4*>(pk);
+    a.ell_val = reinterpret_cast<const float*>(pk);
     a.tc_vals = pk + values_tc_offset(plan, hd.n);
     a.tc_vals_head_stride = (long)values_tc_bytes(plan);
   }
@@ -702,9 +732,9 @@ int stile_spmm_values_pack(const StileSpmmPlan* plan, const float* vals, int32_t
   if ((plan->args.tc_n_items && !plan->args.tc_nnz_id) || (plan->args.ell_n_groups && !plan->args.ell_nnz_id))
     return fail(STILE_E_INVALID, "plan was uploaded without nonzero ids");
   uint8_t* pk = static_cast<uint8_t*>(packed);
-  cudaError_t e = stile::launch_pack_values(plan->args, vals, plan->nnz, heads, pk, pk + values_tc_offset(plan, heads),
-                                            plan->ell_n_slots, (long)values_tc_bytes(plan),
-                                            static_cast<cudaStream_t>(stream));
+  cudaError_t e = stile::launch_pack_values(plan->args, vals, plan->nnz, heads, reinterpret_cast<float*>(pk),
+                                            pk + values_tc_offset(plan, heads), plan->ell_n_slots,
+                                            (long)values_tc_bytes(plan), false, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "value pack launch");
   g_launches++;
   return STILE_OK;
@@ -779,26 +809,30 @@ int stile_spmm_plan_set_transpose_ids(StileSpmmPlan* plan, const int32_t* perm, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const long n_ell = plan->args.ell_n_groups ? plan->ell_n_slots : 0, n_dv = plan->args.dv_n;
   const long n_tc = plan->args.tcdv_n_units ? (long)plan->args.tc_n_ksteps * 256 : 0;
+  const long n_live = plan->n_tc_live;
+  // the ELL ids first: they are read 16 bytes at a time
+  const long o_dv = (n_ell + 3) / 4 * 4, o_tc = o_dv + n_dv, o_live = o_tc + n_tc;
   if (!plan->tid_buf) {
-    cudaError_t e = cudaMalloc(&plan->tid_buf, (size_t)(n_ell + n_dv + n_tc + 1) * 4);
+    cudaError_t e = cudaMalloc(&plan->tid_buf, (size_t)(o_live + n_live + 1) * 4);
     if (e != cudaSuccess) {
       plan->tid_buf = nullptr;
       return cuda_fail(e, "cudaMalloc(transpose ids)");
     }
   }
   int* ids = static_cast<int*>(plan->tid_buf);
-  // the ELL records carry their id in their fourth word; the run list gets
-  // a permuted copy
-  cudaError_t e = stile::launch_record_ids(const_cast<int4*>(plan->args.ell_entry), plan->args.ell_nnz_id, n_ell,
-                                           perm, st);
-  if (e == cudaSuccess) e = stile::launch_permute_ids(plan->args.dv_id, n_dv, perm, ids + n_ell, st);
-  if (e == cudaSuccess && n_tc)
-    e = stile::launch_permute_ids(plan->args.tc_nnz_id, n_tc, perm, ids + n_ell + n_dv, st);
+  // permuted copies of the row-tile entries', the run list's, the k-steps'
+  // and the live elements' ids
+  cudaError_t e = stile::launch_permute_ids(plan->args.ell_nnz_id, n_ell, perm, ids, st);
+  if (e == cudaSuccess) e = stile::launch_permute_ids(plan->args.dv_id, n_dv, perm, ids + o_dv, st);
+  if (e == cudaSuccess) e = stile::launch_permute_ids(plan->args.tc_nnz_id, n_tc, perm, ids + o_tc, st);
+  if (e == cudaSuccess) e = stile::launch_permute_ids(plan->args.tc_live_id, n_live, perm, ids + o_live, st);
   if (e != cudaSuccess) return cuda_fail(e, "id permutation launch");
-  g_launches += (n_ell > 0) + (n_dv > 0) + (n_tc > 0);
-  plan->args.ell_ids_set = 1;
-  plan->args.dvp_id = ids + n_ell;
-  if (n_tc) plan->args.tcdv_id = ids + n_ell + n_dv;
+  g_launches += (n_ell > 0) + (n_dv > 0) + (n_tc > 0) + (n_live > 0);
+  plan->args.ell_fid = ids;
+  plan->args.tc_live_fid = ids + o_live;
+  plan->args.dvp_id = ids + o_dv;
+  if (n_tc) plan->args.tcdv_id = ids + o_tc;
+  plan->ids_set = true;
   return STILE_OK;
 }
 
@@ -846,7 +880,7 @@ int stile_spmm_backward(const StileSpmmPlan* planT, const float* dC, int64_t ldd
   if (!planT) return fail(STILE_E_INVALID, "null plan");
   if (N <= 0) return fail(STILE_E_INVALID, "N must be positive");
   if (!dvals) return fail(STILE_E_INVALID, "null dvals");
-  if (!planT->args.dvp_id || (planT->args.ell_n_groups && !planT->args.ell_ids_set))
+  if (!planT->ids_set)
     return fail(STILE_E_INVALID, "call stile_spmm_plan_set_transpose_ids first");
   int rc;
   if ((rc = check_dense(lddc, N, dC, "dC")) != 0) return rc;
@@ -894,7 +928,7 @@ int stile_spmm_backward(const StileSpmmPlan* planT, const float* dC, int64_t ldd
   return STILE_OK;
 }
 
-int stile_spmm_plan_set_values(StileSpmmPlan* plan, const float* vals, void* stream) {
+static int set_values(StileSpmmPlan* plan, const float* vals, bool forward_ids, void* stream) {
   stile::begin_call();
   if (!plan || !vals) return fail(STILE_E_INVALID, "null argument");
   if (plan->args.tc_n_chunks && plan->args.tc_mode == STILE_TC_FP8)
@@ -902,11 +936,21 @@ int stile_spmm_plan_set_values(StileSpmmPlan* plan, const float* vals, void* str
   if ((plan->args.tc_n_items && !plan->args.tc_nnz_id) ||
       (plan->args.ell_n_groups && !plan->args.ell_nnz_id))
     return fail(STILE_E_INVALID, "plan was uploaded without nonzero ids");
-  cudaError_t e = stile::launch_repack(plan->args, vals, plan->ell_n_slots,
-                                       static_cast<cudaStream_t>(stream));
+  if (forward_ids && !plan->ids_set) return fail(STILE_E_INVALID, "call stile_spmm_plan_set_transpose_ids first");
+  cudaError_t e = stile::launch_pack_values(plan->args, vals, plan->nnz, 1, const_cast<float*>(plan->args.ell_val),
+                                            const_cast<void*>(plan->args.tc_vals), plan->ell_n_slots, 0, forward_ids,
+                                            static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "value re-pack launch");
   g_launches++;
   return STILE_OK;
+}
+
+int stile_spmm_plan_set_values(StileSpmmPlan* plan, const float* vals, void* stream) {
+  return set_values(plan, vals, false, stream);
+}
+
+int stile_spmm_plan_set_values_forward(StileSpmmPlan* planT, const float* vals, void* stream) {
+  return set_values(planT, vals, true, stream);
 }
 
 int stile_spmm_plan_error_flag(StileSpmmPlan* plan, void* stream, int32_t* flag) {

@@ -16,7 +16,7 @@
 //  * dvals               value gradient <dY[row], B[col]> for every nonzero,
 //                        over an entry list built from the same tiles (the
 //                        SDDMM entry-list kernel of sddmm.cu)
-//  * pack_values_kernel  per-head value sets of a batched run
+//  * pack_values_kernel  the tile values from CSR-ordered values (refresh, batched sets)
 #include "common.cuh"
 #include <algorithm>
 #include <map>
@@ -581,8 +581,9 @@ __global__ void __launch_bounds__(kWsThreads, WsCfg<MODE, kIn16>::kCtas) spmm_tc
   if (warp == 0) tmem_dealloc(tmem, 16 * kAccBufs);
 }
 
-// ELL tiles as a stream of live entries in row order, packed as 16-byte
-// records {column, value, 2 * row code + run end, 0}.  An LPR-lane
+// ELL tiles as a stream of live entries in row order: records {column,
+// 2 * row code + run end} and, apart from them, the values (a refresh of the
+// values then writes 4 contiguous bytes an entry).  An LPR-lane
 // sub-group owns one group of <= kSegNnz entries; each lane covers 4 * VEC
 // features of a row, float4 w at features 4 (w LPR + lane), so that every
 // load instruction of the sub-group reads 16 LPR contiguous bytes (whole
@@ -601,7 +602,16 @@ __global__ void __launch_bounds__(kWsThreads, WsCfg<MODE, kIn16>::kCtas) spmm_tc
 // kOff32: every B row offset col * ldb fits in 32 bits.
 // kSpanY: blockIdx.y takes features [y span, (y + 1) span) (a wide B over
 // few groups; span = p.ell_fc_span, a multiple of the pass width).
-// kHeads: a batched run (blockIdx.z = head offsets B, C and the records).
+// kHeads: a batched run (blockIdx.z = head offsets B, C and the values).
+//
+// entry i of a group of n as {column, value bits, 2 * row code + run end};
+// past the group: column 0, value 0, no run end
+__device__ __forceinline__ int3 ell_record(const int2* __restrict__ ent, const float* __restrict__ val, int i, int n) {
+  if (i >= n) return make_int3(0, 0, 0);
+  const int2 e = __ldcs(ent + i);
+  return make_int3(e.x, __float_as_int(__ldcs(val + i)), e.y);
+}
+
 template <int LPR, int VEC, bool kFull, bool kOff32, bool kSpanY = false, bool kHeads = false>
 __global__ void __launch_bounds__(256, 5) spmm_ell_seg_kernel(SpmmArgs p) {
   constexpr int kBatch = 4 / VEC;  // entries per batch: 4 float4 in flight per lane
@@ -623,11 +633,12 @@ __global__ void __launch_bounds__(256, 5) spmm_ell_seg_kernel(SpmmArgs p) {
   const int p0 = __ldg(p.ell_group_ptr + g);
   const int n = __ldg(p.ell_group_ptr + g + 1) - p0;
   const long head = kHeads ? blockIdx.z : 0;
-  const int4* __restrict__ ent = p.ell_entry + head * p.ell_n_pos + p0;
+  const int2* __restrict__ ent = p.ell_entry + p0;
+  const float* __restrict__ val = p.ell_val + head * p.ell_n_pos + p0;
   const int N = p.N;
   const int ldb32 = (int)p.ldb;
   // records are read once: streaming loads leave L2 to the B rows
-  auto rec = [&](int i) { return i < n ? __ldcs(ent + i) : make_int4(0, 0, 0, 0); };
+  auto rec = [&](int i) { return ell_record(ent, val, i, n); };
   for (int fc = kSpanY ? blockIdx.y * p.ell_fc_span : 0;
        fc < (kSpanY ? min(N, (int)(blockIdx.y + 1) * p.ell_fc_span) : N); fc += 4 * VEC * LPR) {
     // float4 w of this lane holds features f + 4 LPR w: each load
@@ -637,10 +648,10 @@ __global__ void __launch_bounds__(256, 5) spmm_ell_seg_kernel(SpmmArgs p) {
     float4 acc[VEC];
 #pragma unroll
     for (int w = 0; w < VEC; ++w) acc[w] = make_float4(0.f, 0.f, 0.f, 0.f);
-    int4 mcur = rec(sl);
+    int3 mcur = rec(sl);
 #pragma unroll 1
     for (int c0 = 0; c0 < n; c0 += LPR) {
-      const int4 mnext = rec(c0 + LPR + sl);
+      const int3 mnext = rec(c0 + LPR + sl);
 #pragma unroll 1
       for (int b0 = c0; b0 < min(n, c0 + LPR); b0 += kBatch) {
         float4 bv[kBatch][VEC];
@@ -695,7 +706,7 @@ __global__ void __launch_bounds__(256, 5) spmm_ell_seg_kernel(SpmmArgs p) {
 // (N <= 8 LPR), and for every entry (row r, column c) of A^T also
 //   dv_out[id] = <dC[c], dvx[r]>,
 // the value gradient of the forward's nonzero (c, r); id, in the forward's
-// numbering, rides in the entry record's fourth word.  The dC row gathered
+// numbering, comes with the entry (ell_fid).  The dC row gathered
 // for the product is the one the gradient needs; dvx[r] (the forward's
 // dense operand) is loaded where a row run starts, for both entries of a
 // batch before either is used, so those loads overlap the dC gathers.  The
@@ -716,12 +727,17 @@ __global__ void __launch_bounds__(256, 4) spmm_ell_bwd_kernel(SpmmArgs p) {
   }
   const int p0 = __ldg(p.ell_group_ptr + g);
   const int n = __ldg(p.ell_group_ptr + g + 1) - p0;
-  const int4* __restrict__ ent = p.ell_entry + p0;
+  const int2* __restrict__ ent = p.ell_entry + p0;
+  const float* __restrict__ val = p.ell_val + p0;
+  const int* __restrict__ fid = p.ell_fid + p0;
   const int N = p.N;
   // this lane's features: f .. f + 3 and f + 4 LPR .. f + 4 LPR + 3 (each
   // load instruction of the group reads 16 LPR contiguous bytes of a row)
   const int f = 4 * sl, f2 = f + 4 * LPR;
-  auto rec = [&](int i) { return i < n ? __ldcs(ent + i) : make_int4(0, 0, 0, -1); };
+  auto rec = [&](int i) {
+    const int3 r = ell_record(ent, val, i, n);
+    return make_int4(r.x, r.y, r.z, i < n ? __ldcs(fid + i) : -1);
+  };
   auto row_of = [](int ce) { const int code = ce >> 1; return code >= 0 ? code : -code - 1; };
   auto ld8 = [&](const float* row, float4& a, float4& b) {
     a = kFull ? ldg4(row + f) : ld4_live(row, f, N);
@@ -800,22 +816,6 @@ __global__ void __launch_bounds__(256, 4) spmm_ell_bwd_kernel(SpmmArgs p) {
   if (p.ell_lazy_wait) griddep_wait();
 }
 
-// fourth word of every ELL record := the forward operator's id of its
-// nonzero (perm of the record's own id), -1 for padding
-__global__ void record_ids_kernel(int4* __restrict__ ent, const int* __restrict__ ids, long n,
-                                  const int* __restrict__ perm) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int v = ids[i];
-  ent[i].w = v >= 0 ? perm[v] : -1;
-}
-
-cudaError_t launch_record_ids(int4* ent, const int* ids, long n, const int* perm, cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  record_ids_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ent, ids, n, perm);
-  return cudaGetLastError();
-}
-
 __global__ void permute_ids_kernel(const int* __restrict__ in, long n, const int* __restrict__ perm,
                                    int* __restrict__ out) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -854,21 +854,22 @@ __global__ void __launch_bounds__(256, 4) spmm_ell_seg_bf16_kernel(SpmmArgs p) {
   }
   const int p0 = __ldg(p.ell_group_ptr + g);
   const int n = __ldg(p.ell_group_ptr + g + 1) - p0;
-  const int4* __restrict__ ent = p.ell_entry + blockIdx.z * p.ell_n_pos + p0;
+  const int2* __restrict__ ent = p.ell_entry + p0;
+  const float* __restrict__ val = p.ell_val + blockIdx.z * p.ell_n_pos + p0;
   const uint16_t* __restrict__ B16 = reinterpret_cast<const uint16_t*>(p.B) + blockIdx.z * p.b_head_stride;
   float* __restrict__ Ch = p.C + blockIdx.z * p.c_head_stride;
   const int N = p.N;
   const int ldb32 = (int)p.ldb;
   // records are read once: streaming loads leave L2 to the B rows
-  auto rec = [&](int i) { return i < n ? __ldcs(ent + i) : make_int4(0, 0, 0, 0); };
+  auto rec = [&](int i) { return ell_record(ent, val, i, n); };
   for (int fc = kSpanY ? blockIdx.y * p.ell_fc_span : 0;
        fc < (kSpanY ? min(N, (int)(blockIdx.y + 1) * p.ell_fc_span) : N); fc += 8 * LPR) {
     const int f = fc + 8 * sl;
     float4 acc0 = make_float4(0.f, 0.f, 0.f, 0.f), acc1 = acc0;
-    int4 mcur = rec(sl);
+    int3 mcur = rec(sl);
 #pragma unroll 1
     for (int c0 = 0; c0 < n; c0 += LPR) {
-      const int4 mnext = rec(c0 + LPR + sl);
+      const int3 mnext = rec(c0 + LPR + sl);
 #pragma unroll 1
       for (int b0 = c0; b0 < min(n, c0 + LPR); b0 += kBatch) {
         uint4 bv[kBatch];
@@ -923,74 +924,82 @@ __global__ void __launch_bounds__(256, 4) spmm_ell_seg_bf16_kernel(SpmmArgs p) {
 // ===========================================================================
 
 // ===========================================================================
-// value re-pack: refresh the plan's tile values from a CSR-ordered value
-// array (used when the matrix values change but the pattern does not)
+// value refresh: the plan's tile values from CSR-ordered value arrays (new
+// values on the same pattern; the value sets of a batched run)
 // ===========================================================================
-__global__ void repack_values_kernel(SpmmArgs p, const float* __restrict__ vals, int4* ell_entry,
-                                     uint16_t* tc_img, long n_ell_slots) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long n_tc = (long)p.tc_n_ksteps * 256;
-  if (i < n_tc) {
-    const long ks = i >> 8;
-    const int e = (int)(i & 255), n = e >> 4, k = e & 15;
-    const int id = p.tc_nnz_id[i];
-    const float v = id >= 0 ? vals[id] : 0.f;
-    const int img = (n >> 3) * 128 + (k >> 3) * 64 + (n & 7) * 8 + (k & 7);
-    if (p.tc_mode == STILE_TC_F16) {
-      __half h = __float2half_rn(v);
-      tc_img[ks * 256 + img] = *reinterpret_cast<uint16_t*>(&h);
-    } else {
-      __nv_bfloat16 h = __float2bfloat16_rn(v);
-      if (p.tc_mode == STILE_TC_SPLIT_BF16) {
-        __nv_bfloat16 l = __float2bfloat16_rn(v - __bfloat162float(h));
-        tc_img[ks * 512 + img] = *reinterpret_cast<uint16_t*>(&h);
-        tc_img[ks * 512 + 256 + img] = *reinterpret_cast<uint16_t*>(&l);
-      } else {
-        tc_img[ks * 256 + img] = *reinterpret_cast<uint16_t*>(&h);
-      }
-    }
-  } else if (i - n_tc < n_ell_slots) {
-    const long s = i - n_tc;
-    const int id = p.ell_nnz_id[s];
-    ell_entry[s].y = __float_as_int(id >= 0 ? vals[id] : 0.f);
-  }
-}
-
-// Value sets of a batched run: for head blockIdx.y, the tensor-tile images
-// (in the plan's k-step order and mode) and the ELL records (the plan's
-// column and row code, the head's value) built from vals + head * nnz.
-__global__ void pack_values_kernel(SpmmArgs p, const float* __restrict__ vals, long nnz, int4* __restrict__ ell_out,
-                                   uint16_t* __restrict__ tc_out, long n_ell, long tc_head_elems) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+// Bound by memory: it reads every value once (a 32-byte sector per value,
+// their order is the tiles', not the CSR's) and writes every tile value.  A
+// warp takes one k-step of a tensor tile: lane l owns the 8 image elements
+// 8l .. 8l + 7, a byte of the k-step's mask says which of them hold a
+// nonzero, their ids lie one after another, and the lane writes its 16 bytes
+// of the image at once (the other elements are zero).  The ids of the dead
+// elements are never read: a k-step of the 233k-node graph holds 41 nonzeros
+// of 256, 196 bytes of mask and ids in place of 1 KB.  The row-tile values
+// are an array of their own, 4 entries a thread.
+constexpr int kPackThreads = 256;
+template <int MODE>
+__global__ void __launch_bounds__(kPackThreads) pack_values_kernel(SpmmArgs p, const float* __restrict__ vals, long nnz,
+                                                                   const int* __restrict__ tc_ids,
+                                                                   const int* __restrict__ ell_ids,
+                                                                   float* __restrict__ ell_out,
+                                                                   uint8_t* __restrict__ tc_out, long n_ell,
+                                                                   long tc_head_bytes, int tc_blocks) {
   const long h = blockIdx.y;
-  const float* hv = vals + h * nnz;
-  const long n_tc = (long)p.tc_n_ksteps * 256;
-  if (i < n_tc) {
-    const long ks = i >> 8;
-    const int e = (int)(i & 255), n = e >> 4, k = e & 15;
-    const int id = p.tc_nnz_id[i];
-    const float v = id >= 0 ? hv[id] : 0.f;
-    const int img = (n >> 3) * 128 + (k >> 3) * 64 + (n & 7) * 8 + (k & 7);
-    uint16_t* out = tc_out + h * tc_head_elems;
-    if (p.tc_mode == STILE_TC_F16) {
-      __half x = __float2half_rn(v);
-      out[ks * 256 + img] = *reinterpret_cast<uint16_t*>(&x);
+  const float* __restrict__ hv = vals + h * nnz;
+  if ((int)blockIdx.x < tc_blocks) {
+    const int ks = blockIdx.x * (kPackThreads / kWarp) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (ks >= p.tc_n_ksteps) return;
+    const unsigned m = __ldg(p.tc_live_mask + (long)ks * 32 + lane);
+    int before = __popc(m);  // inclusive scan of the lanes' counts
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += v;
+    }
+    const int* ids = tc_ids + __ldg(p.tc_live_ptr + ks) + before - __popc(m);
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const bool live = (m >> j) & 1u;
+      v[j] = live ? __ldg(hv + __ldcs(ids + __popc(m & ((1u << j) - 1u)))) : 0.f;
+    }
+    constexpr uint32_t kBytes = MODE == STILE_TC_SPLIT_BF16 ? 2 * kBStage : kBStage;
+    uint4* out = reinterpret_cast<uint4*>(tc_out + h * tc_head_bytes + (long)ks * kBytes) + lane;
+    if constexpr (MODE == STILE_TC_F16) {
+      *out = make_uint4(pack_f16x2(v[0], v[1]), pack_f16x2(v[2], v[3]), pack_f16x2(v[4], v[5]), pack_f16x2(v[6], v[7]));
     } else {
-      __nv_bfloat16 x = __float2bfloat16_rn(v);
-      if (p.tc_mode == STILE_TC_SPLIT_BF16) {
-        __nv_bfloat16 l = __float2bfloat16_rn(v - __bfloat162float(x));
-        out[ks * 512 + img] = *reinterpret_cast<uint16_t*>(&x);
-        out[ks * 512 + 256 + img] = *reinterpret_cast<uint16_t*>(&l);
-      } else {
-        out[ks * 256 + img] = *reinterpret_cast<uint16_t*>(&x);
+      uint32_t hi[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) hi[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+      *out = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      if constexpr (MODE == STILE_TC_SPLIT_BF16) {
+        uint32_t lo[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          lo[j] = pack_bf16x2(v[2 * j] - __uint_as_float(hi[j] << 16),
+                              v[2 * j + 1] - __uint_as_float(hi[j] & 0xffff0000u));
+        out[kBStage / 16] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
       }
     }
-  } else if (i - n_tc < n_ell) {
-    const long s = i - n_tc;
-    const int id = p.ell_nnz_id[s];
-    int4 r = p.ell_entry[s];
-    r.y = __float_as_int(id >= 0 ? hv[id] : 0.f);
-    ell_out[h * n_ell + s] = r;
+    return;
+  }
+  const long i = 4 * ((long)(blockIdx.x - tc_blocks) * kPackThreads + threadIdx.x);
+  float* __restrict__ out = ell_out + h * n_ell;
+  auto value = [&](int id) { return id >= 0 ? __ldg(hv + id) : 0.f; };
+  if (i + 4 <= n_ell) {
+    // the ids are 16-byte aligned; a head's values only when n_ell % 4 == 0
+    const int4 id = __ldcs(reinterpret_cast<const int4*>(ell_ids + i));
+    const float4 v = make_float4(value(id.x), value(id.y), value(id.z), value(id.w));
+    if (((h * n_ell) & 3) == 0) {
+      *reinterpret_cast<float4*>(out + i) = v;
+    } else {
+      out[i] = v.x;
+      out[i + 1] = v.y;
+      out[i + 2] = v.z;
+      out[i + 3] = v.w;
+    }
+  } else {
+    for (long j = i; j < n_ell; ++j) out[j] = value(__ldg(ell_ids + j));
   }
 }
 
@@ -1015,22 +1024,20 @@ cudaError_t launch_amax(const float* B, long ldb, int K, int N, unsigned* amax_b
   return cudaGetLastError();
 }
 
-cudaError_t launch_pack_values(const SpmmArgs& p, const float* vals, long nnz, int heads, void* ell_out,
-                               void* tc_out, long n_ell, long tc_head_bytes, cudaStream_t st) {
-  const long total = (long)p.tc_n_ksteps * 256 + n_ell;
-  if (total == 0 || heads == 0) return cudaSuccess;
-  pack_values_kernel<<<dim3((unsigned)((total + 255) / 256), heads), 256, 0, st>>>(
-      p, vals, nnz, static_cast<int4*>(ell_out), static_cast<uint16_t*>(tc_out), n_ell, tc_head_bytes / 2);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_repack(const SpmmArgs& p, const float* vals, long n_ell_slots, cudaStream_t st) {
-  const long total = (long)p.tc_n_ksteps * 256 + n_ell_slots;
-  if (total == 0) return cudaSuccess;
-  const long grid = (total + 255) / 256;
-  repack_values_kernel<<<(unsigned)grid, 256, 0, st>>>(
-      p, vals, const_cast<int4*>(p.ell_entry),
-      reinterpret_cast<uint16_t*>(const_cast<void*>(p.tc_vals)), n_ell_slots);
+cudaError_t launch_pack_values(const SpmmArgs& p, const float* vals, long nnz, int heads, float* ell_out,
+                               void* tc_out, long n_ell, long tc_head_bytes, bool forward_ids, cudaStream_t st) {
+  constexpr int kWarps = kPackThreads / kWarp;
+  const int tc_blocks = (p.tc_n_ksteps + kWarps - 1) / kWarps;
+  const long ell_blocks = (n_ell + 4 * kPackThreads - 1) / (4 * kPackThreads);
+  if (tc_blocks + ell_blocks == 0 || heads == 0) return cudaSuccess;
+  const int* tc_ids = forward_ids ? p.tc_live_fid : p.tc_live_id;
+  const int* ell_ids = forward_ids ? p.ell_fid : p.ell_nnz_id;
+  const dim3 grid((unsigned)(tc_blocks + ell_blocks), (unsigned)heads);
+  auto k = p.tc_mode == STILE_TC_F16            ? pack_values_kernel<STILE_TC_F16>
+           : p.tc_mode == STILE_TC_SPLIT_BF16 ? pack_values_kernel<STILE_TC_SPLIT_BF16>
+                                              : pack_values_kernel<STILE_TC_BF16>;
+  k<<<grid, kPackThreads, 0, st>>>(p, vals, nnz, tc_ids, ell_ids, ell_out, static_cast<uint8_t*>(tc_out), n_ell,
+                                   tc_head_bytes, tc_blocks);
   return cudaGetLastError();
 }
 

@@ -17,8 +17,8 @@ struct SpmmArgs {
   int ell_lazy_wait;  // the ELL kernel's predecessor is the zero-rows kernel: only its adds wait
   // heads of a batched run (blockIdx.z; 0 and unused otherwise): per head, B
   // and C start head * stride elements further, the value images head *
-  // tc_vals_head_stride bytes further and the ELL records head * ell_n_pos
-  // records further
+  // tc_vals_head_stride bytes further and the ELL values head * ell_n_pos
+  // values further
   long b_head_stride, c_head_stride, tc_vals_head_stride;
   int heads;  // grid.z of the ELL and tensor-core launches (0 or 1: one head)
   int tc_slice_per;      // 128-feature slices per tensor-core CTA (blockIdx.y); set by the launcher
@@ -47,6 +47,15 @@ struct SpmmArgs {
   const int* tc_cols;
   const void* tc_vals;
   const int* tc_nnz_id;
+  // live elements of the value images, k-step by k-step: bit i of the 256-bit
+  // mask of k-step ks (32 bytes, element i in image order) is set when the
+  // element holds a nonzero; the nonzeros' ids, in image order, are
+  // tc_live_id[tc_live_ptr[ks] ..]; tc_live_fid: the same in the forward
+  // operator's numbering (set_transpose_ids)
+  const uint8_t* tc_live_mask;
+  const int* tc_live_ptr;
+  const int* tc_live_id;
+  const int* tc_live_fid;
   // STILE_TC_FP8: scale of every (item, row) and the device word that holds
   // the bits of max |B| of the run (written by an amax pass before the
   // kernels; B's e4m3 scale is that / 448)
@@ -58,11 +67,13 @@ struct SpmmArgs {
   int ell_n_groups;
   long ell_n_pos;
   const int* ell_group_ptr;  // [ell_n_groups + 1]
-  // [ell_n_pos] {column of B, value bits, 2 * row code + run end, 0}; row
-  // code r stores into C row r, -(r + 1) adds; run end is 1 when the entry
-  // ends its row's run in the group
-  const int4* ell_entry;
+  // [ell_n_pos] {column of B, 2 * row code + run end}; row code r stores into
+  // C row r, -(r + 1) adds; run end is 1 when the entry ends its row's run in
+  // the group
+  const int2* ell_entry;
+  const float* ell_val;      // [ell_n_pos] values ([heads * ell_n_pos] of a batched run)
   const int* ell_nnz_id;     // [ell_n_pos] nonzero id (or NULL)
+  const int* ell_fid;        // [ell_n_pos] the same in the forward's numbering (set_transpose_ids)
   // value-gradient entry list enumerated from the tiles: tensor-core entries
   // (item, row, k-step, column order) then ELL slots (row, slot order)
   long dv_n;
@@ -86,14 +97,13 @@ struct SpmmArgs {
   int stall_test;
   // fused backward (this plan is the transposed operator's): the ELL pass
   // that computes dB = A^T dC also writes dvals[id] = <dC[col], dvx[row]>
-  // for its entries, id in the fourth word of each record (dvx: the
-  // forward's dense operand), and the run list's tensor-core prefix
-  // (dv_n_groups_tc groups) gives the rest with ids dvp_id; ids in the
-  // forward operator's nonzero numbering (set by set_transpose_ids)
+  // for its entries, id from ell_fid (dvx: the forward's dense operand), and
+  // the run list's tensor-core prefix (dv_n_groups_tc groups) gives the rest
+  // with ids dvp_id; ids in the forward operator's nonzero numbering (set by
+  // set_transpose_ids)
   const float* dvx;
   long dvx_ld;
   float* dv_out;
-  int ell_ids_set;
   const int* dvp_id;
   int dv_n_groups_tc;
   // value gradients of the tensor-tile nonzeros on the tensor cores: units
@@ -132,8 +142,6 @@ cudaError_t launch_ell(const SpmmArgs& p, cudaStream_t st);
 cudaError_t launch_ell_bwd(const SpmmArgs& p, cudaStream_t st);
 // out[i] = in[i] >= 0 ? perm[in[i]] : -1
 cudaError_t launch_permute_ids(const int* in, long n, const int* perm, int* out, cudaStream_t st);
-// ent[i].w = ids[i] >= 0 ? perm[ids[i]] : -1
-cudaError_t launch_record_ids(int4* ent, const int* ids, long n, const int* perm, cudaStream_t st);
 cudaError_t launch_dvals(const SpmmArgs& p, const float* dY, long lddy, float* dvals, cudaStream_t st);
 // out[id] = <X[item row], Y[k-step column]> for the tensor-tile nonzeros
 // (fp32 X and Y, F features), on the tensor cores with hi + lo bf16
@@ -142,9 +150,11 @@ cudaError_t launch_tc_dvals(const SpmmArgs& p, const float* X, long ldx, const f
                             cudaStream_t st);
 constexpr int kTcDvUnit = 8;  // k-steps per unit of the tensor-tile value-gradient kernel
 constexpr int kChunkSteps = 32;
-cudaError_t launch_pack_values(const SpmmArgs& p, const float* vals, long nnz, int heads, void* ell_out,
-                               void* tc_out, long n_ell, long tc_head_bytes, cudaStream_t st);
-cudaError_t launch_repack(const SpmmArgs& p, const float* vals, long n_ell_slots, cudaStream_t st);
+// the tile values of `heads` value sets (vals + h * nnz) into ell_out (+ h *
+// n_ell values) and the tensor-tile images tc_out (+ h * tc_head_bytes);
+// forward_ids: vals are in the forward operator's numbering
+cudaError_t launch_pack_values(const SpmmArgs& p, const float* vals, long nnz, int heads, float* ell_out,
+                               void* tc_out, long n_ell, long tc_head_bytes, bool forward_ids, cudaStream_t st);
 // *amax_bits = bits of max |B[r][f]| over K rows x N features (atomicMax on
 // the non-negative floats' bits; *amax_bits starts at 0); an ordinary launch
 cudaError_t launch_amax(const float* B, long ldb, int K, int N, unsigned* amax_bits, cudaStream_t st);

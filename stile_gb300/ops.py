@@ -302,6 +302,16 @@ class DeviceSpmmPlan:
         _lib.check(self.lib.stile_spmm_plan_set_values(self.handle, vals.data_ptr(), _stream()),
                    "stile_spmm_plan_set_values")
 
+    def set_values_forward(self, vals: torch.Tensor):
+        """Values of A, in A's numbering, into this plan of A^T (after
+        set_transpose_ids)."""
+        _require_cuda(vals, "vals")
+        vals = vals.float().contiguous()
+        if vals.numel() != self.nnz:
+            raise ValueError("vals must have one entry per nonzero")
+        _lib.check(self.lib.stile_spmm_plan_set_values_forward(self.handle, vals.data_ptr(), _stream()),
+                   "stile_spmm_plan_set_values_forward")
+
     def set_wait_policy(self, polls: int = 0, stall_test: bool = False):
         """Poll limit of the tensor-core kernel's pipeline waits (0: the
         default) and the failure-detection stall test
