@@ -469,16 +469,33 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
       }
   if ((long)h->tc_n_items * stile::kTcDvUnit > INT32_MAX) return fail(STILE_E_INVALID, "too many tensor-tile items");
 
+  // the units of every chunk (what the kernel reads of them), the unit of
+  // every k-step within its CTA, and every CTA's units and k-steps
+  std::vector<int32_t> un_meta, un_rows, un_item, step_unit, cta_info;
+  for (int b = 0; b < tc_grid; ++b) {
+    const int u0 = (int)un_meta.size(), k0 = (int)step_unit.size();
+    for (int c = cta_chunk[b]; c < cta_chunk[b + 1]; ++c) {
+      const int per = mode == STILE_TC_SPLIT_BF16 ? stile::kSplitSteps : stile::kChunkSteps;
+      for (int o = 0; o < ck_nk[c]; o += per) {
+        const int n = std::min(per, ck_nk[c] - o);
+        step_unit.insert(step_unit.end(), n, (int)un_meta.size() - u0);
+        un_meta.push_back(n | (ck_flags[c] ? stile::kUnitAdds : 0) | (o == 0 ? stile::kUnitFirst : 0) |
+                          (o + n == ck_nk[c] ? stile::kUnitLast : 0));
+        un_item.push_back(ck_item[c]);
+        un_rows.insert(un_rows.end(), h->tc_out_rows + (long)ck_item[c] * 16, h->tc_out_rows + (long)ck_item[c] * 16 + 16);
+      }
+    }
+    cta_info.insert(cta_info.end(), {u0, (int)un_meta.size() - u0, k0, (int)step_unit.size() - k0});
+  }
+
   Arena ar;
-  const long ti = h->tc_n_items, tk = h->tc_n_ksteps;
-  size_t i_kbeg = ar.add(h->tc_item_kbeg, ti ? (ti + 1) * 4 : 0);
-  size_t i_flags = ar.add(h->tc_item_flags, ti * 4);
+  const long ti = h->tc_n_items;
   size_t i_orows = ar.add(h->tc_out_rows, ti * 16 * 4);
   // k-step arrays in schedule order (every k-step belongs to exactly one chunk)
   size_t i_cols = ar.add(s_cols.data(), s_cols.size() * 4);
   size_t i_vals = ar.add(s_vals.data(), s_vals.size());
   size_t i_tnid = ar.add(s_nnz.data(), s_nnz.size() * 4);
-  size_t i_ctac = ar.add(cta_chunk.data(), cta_chunk.size() * 4);
+  size_t i_ctai = ar.add(cta_info.data(), cta_info.size() * 4);
   size_t i_egptr = ar.add(e_gptr.data(), e_gptr.size() * 4);
   size_t i_eent = ar.add(e_ent.data(), e_ent.size() * 4);
   size_t i_eval = ar.add(e_val.data(), e_val.size() * 4);
@@ -487,10 +504,10 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
   size_t i_lid = ar.add(live_id.data(), live_id.size() * 4);
   size_t i_enid = ar.add(e_id.data(), e_id.size() * 4);
   size_t i_zero = ar.add(zero.data(), zero.size() * 4);
-  size_t i_ckb = ar.add(ck_kbeg.data(), (size_t)nck * 4);
-  size_t i_ckn = ar.add(ck_nk.data(), (size_t)nck * 4);
-  size_t i_cki = ar.add(ck_item.data(), (size_t)nck * 4);
-  size_t i_ckf = ar.add(ck_flags.data(), (size_t)nck * 4);
+  size_t i_unm = ar.add(un_meta.data(), un_meta.size() * 4);
+  size_t i_unr = ar.add(un_rows.data(), un_rows.size() * 4);
+  size_t i_uni = ar.add(un_item.data(), un_item.size() * 4);
+  size_t i_stu = ar.add(step_unit.data(), step_unit.size() * 4);
   size_t i_dvr = ar.add(dv_row.data(), (size_t)ndv * 4);
   size_t i_dvc = ar.add(dv_col.data(), (size_t)ndv * 4);
   size_t i_dvi = ar.add(dv_id.data(), (size_t)ndv * 4);
@@ -533,8 +550,6 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
   a.K = h->K;
   a.tc_n_items = h->tc_n_items;
   a.tc_n_ksteps = h->tc_n_ksteps;
-  a.tc_item_kbeg = (const int*)P(i_kbeg);
-  a.tc_item_flags = (const int*)P(i_flags);
   a.tc_out_rows = (const int*)P(i_orows);
   a.tc_cols = (const int*)P(i_cols);
   a.tc_vals = P(i_vals);
@@ -567,13 +582,13 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
   a.dv_n_groups_tc = dv_groups_tc;
   a.dv_gptr = (const int*)P(i_dvgp);
   a.dv_grow = (const int*)P(i_dvgr);
-  a.tc_chunk_kbeg = (const int*)P(i_ckb);
-  a.tc_chunk_nk = (const int*)P(i_ckn);
+  a.tc_unit_meta = (const int*)P(i_unm);
+  a.tc_unit_rows = (const int*)P(i_unr);
+  a.tc_unit_item = (const int*)P(i_uni);
+  a.tc_step_unit = (const int*)P(i_stu);
   a.tc_grid = tc_grid;
   a.tc_max_cta_steps = (int)max_cta_steps;
-  a.tc_cta_chunk = (const int*)P(i_ctac);
-  a.tc_chunk_item = (const int*)P(i_cki);
-  a.tc_chunk_flags = (const int*)P(i_ckf);
+  a.tc_cta_info = (const int4*)P(i_ctai);
   a.tcdv_n_units = (int)u_ks.size();
   a.tcdv_unit_ks = (const int*)P(i_uks);
   a.tcdv_unit_meta = (const int*)P(i_umeta);

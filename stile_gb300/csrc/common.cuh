@@ -75,6 +75,26 @@ __device__ __forceinline__ void red_row4(float* row, int f, int N, float4 v) {
   }
 }
 
+// *p += v / *p = v where `on`, without a branch (a branch per row cost 35
+// cycles a row in the tensor-core kernel's epilogue); the store is evict
+// first
+__device__ __forceinline__ void red_if(bool on, void* p, float v) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %0, 0;\n\t"
+      "@q red.global.add.f32 [%1], %2;\n\t}\n" ::"r"((int)on),
+      "l"(p), "f"(v)
+      : "memory");
+}
+__device__ __forceinline__ void st_if(bool on, void* p, float v) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %0, 0;\n\t"
+      "@q st.global.cs.f32 [%1], %2;\n\t}\n" ::"r"((int)on),
+      "l"(p), "f"(v)
+      : "memory");
+}
+
 // Programmatic dependent launch: a kernel launched with programmatic stream
 // serialization may start while the previous kernel on the stream drains.
 // griddep_wait() returns once that kernel has completed and its writes are
@@ -325,6 +345,49 @@ __device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t adesc, uint64_
       : "memory");
 }
 
+// The same for code that a whole warp runs: only the lane with `on` set
+// issues.  The operands are then computed uniformly for the warp; inside a
+// one-lane branch every descriptor had to be moved into uniform registers
+// first.
+__device__ __forceinline__ void umma_f16_if(bool on, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((int)on)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f8_if(bool on, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((int)on)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(bool on, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(bar),
+      "r"((int)on)
+      : "memory");
+}
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(on));
+  return on != 0;
+}
+
 // arrive on an mbarrier once all previously issued tcgen05 ops of this thread finish
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile(
@@ -342,6 +405,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+// 32 TMEM lanes x 8 columns of 32 bits -> 8 registers per thread
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");

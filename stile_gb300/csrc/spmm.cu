@@ -2,11 +2,11 @@
 //
 //  * csr_spmm_kernel     plain CSR-row SpMM (the comparator)
 //  * zero_rows_kernel    zeroes output rows that no owned tile stores
-//  * spmm_tc_ws_kernel   dense 16-row block tiles on the tensor cores
-//                        (tcgen05.mma, accumulator in TMEM): warp-specialised
-//                        cp.async producers + MMA issuer (bf16 / fp16, and
-//                        split-bf16 hi+lo products with periodic accumulator
-//                        drains for fp32-level accuracy)
+//  * spmm_tc_kernel      dense 16-row block tiles on the tensor cores
+//                        (tcgen05.mma, accumulator in TMEM): gathering warps
+//                        that hold the rows in registers + an MMA warp (bf16 /
+//                        fp16 / fp8, and split-bf16 hi+lo products with
+//                        periodic accumulator drains for fp32-level accuracy)
 //  * spmm_ell_seg_kernel ELL row-bucket tiles on CUDA cores, as a stream of
 //                        live entries cut into groups at row boundaries
 //                        The two launches together are the reference's
@@ -19,8 +19,10 @@
 //  * pack_values_kernel  the tile values from CSR-ordered values (refresh, batched sets)
 #include "common.cuh"
 #include <algorithm>
+#include <climits>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "spmm.cuh"
 
@@ -149,7 +151,6 @@ constexpr uint32_t kAStage = 4096;   // bytes of one A image (16-bit)
 constexpr uint32_t kBStage = 512;    // bytes of one B image (16-bit)
 constexpr uint32_t kALbo = 2048, kASbo = 1024;
 constexpr uint32_t kBLbo = 128, kBSbo = 256;
-constexpr uint32_t kRawRows = 8192;  // 16 rows x 128 fp32 per stage
 // fp8 operands (K = 32 bytes, K-major, no swizzle): core matrices of 8 rows
 // x 16 bytes, the two k halves 128 B apart (LBO), 8-row groups 256 B apart
 // (SBO); the A image is 4 KB, a k-step's value image 512 B
@@ -162,92 +163,114 @@ __device__ __forceinline__ uint32_t a_img_off(int m, int k) {
   return (uint32_t)(atom * kALbo + grp * kASbo + r * 128 + ((chunk ^ r) << 4) + (m & 7) * 2);
 }
 
-// Persistent bf16 / fp16 tensor-core kernel.
+// Tensor-core kernel.
 //
 // The upload assigns chunks to the kernel's CTAs (longest first, each to the
 // least loaded CTA) and stores every CTA's k-steps contiguously, so a CTA's
 // work is the step range [s_beg, s_beg + S), walked once per 128-feature
-// slice; its units are (slice, chunk) pairs in that order.
-// Roles (kProdWarps producer warps, then one warp whose lane 0 issues the
-// MMAs, then four epilogue warps):
-//  * Producers: warp w fills the steps g = w, w + kProdWarps, ... and owns
-//    raw stage w and operand slot g % kWsSlots.  Per step each lane copies
-//    features 4l..4l+3 of the step's 16 B rows and 16 bytes of its 512-byte
-//    value image with cp.async into the stage (the rows' column ids, one per
-//    lane 0-15, were loaded one step earlier and are broadcast by shuffle),
-//    then, once the copies landed and the MMA that last read the slot has
-//    committed its empty barrier, converts its own copies to the bf16 / fp16
-//    A image in the slot, and lane 0 arrives on the slot's full barrier.
-//    The next step's copies go out right after, so every producer warp keeps
-//    one step in flight while the others convert: the steps of one CTA
-//    overlap kProdWarps ways, and no producer waits on another.
-//  * MMA: per unit t waits until the epilogue released accumulator t % 4
-//    (TMEM columns 16 * (t % 4)), then per step waits for a full slot,
-//    issues tcgen05.mma and commits to the slot's empty barrier; a unit's
-//    last step also commits to the accumulator's full barrier.
-//  * Epilogue: per unit waits for its accumulator, reads it (warp w reads
-//    TMEM lanes 32 * (w % 4)..+31), releases it and writes C.
+// slice; its units are (slice, accumulation unit) pairs in that order.
+//  * Seven gathering warps.  A stage is kSpw consecutive k-steps: 1 at 128
+//    fp32 features a row, 2 or 4 where 64 or 32 features (or 16-bit rows)
+//    leave a warp-wide 16-byte load room for 2 or 4 rows, so every stage is 16
+//    loads of 512 bytes.  Warp w takes the stages w, w + 7, ...  It holds a
+//    stage's rows in registers, converts them into its operand slot (A: the
+//    features are M = 128) and at once loads its next stage's rows, which are
+//    in flight while the MMA warp and the epilogue work.  The rows never pass
+//    through a shared-memory stage: a gathered row costs the L1 / shared
+//    memory pipe its load, half its bytes as operand image and the MMA's read
+//    of that, where the cp.async stage of an earlier build added a write and a
+//    read of the whole fp32 row.  Column ids and value images come by cp.async
+//    two and one stages ahead.
+//    14 gathering warps at 128 registers per SM measured faster than 16 at 96
+//    (spilled) and than 16 warps that each owned accumulators, whose sums also
+//    depended on the split.
+//  * The MMA warp takes the stages in order and accumulates the
+//    k-steps of a unit one after another into one of kAccBufs 16-column
+//    accumulators, so the sums do not depend on the warps' timing.
+//  * Epilogue, by the gathering warps: before its stage in unit y a warp
+//    writes its share (a quarter of the features, half of the tile's rows;
+//    warp 3 both halves) of every unit up to y - kLag - 1, whose MMAs are long
+//    done.
+// Bound by the stages' own chain (wait, convert, issue, fence: about 1,400
+// cycles without contention, 14 of them in turn on an SM), not by L2 or the
+// tensor pipe.  Forward of a graph (row tiles included), before -> after:
+// 169,343 nodes, 1.17M nonzeros: N = 128 64 -> 57 us, N = 41 80 -> 64 us,
+// N = 256 in bf16 121 -> 101 us; 50,000 nodes, 2.4M nonzeros: N = 128 73 -> 62
+// us, N = 41 70 -> 54 us; a 4096^2 matrix in split-bf16 22 -> 12 us; a pruned
+// 3072 x 768 weight at N = 4096 in bf16 223 -> 136 us.
 // Every wait is bounded; a wait that gives up sets the error flag and ends
-// that role, and the others then end at their next (bounded) wait.
-constexpr int kProdWarps = 4;                            // producer warps, one step in flight each
-constexpr int kAccBufs = 4;                              // accumulators of 16 TMEM columns
-constexpr int kWsThreads = (kProdWarps + 1 + 4) * 32;   // producers, MMA warp, 4 epilogue warps
+// that warp's work, and the others then end at their next (bounded) wait.
+constexpr int kTcWarps = 7;                        // gathering warps
+constexpr int kTcThreads = (kTcWarps + 1) * kWarp; // and the MMA warp
+constexpr int kTcCtas = 2;                         // resident CTAs per SM (128 registers a thread)
+constexpr int kAccBufs = 8;                        // accumulators of 16 TMEM columns
+// units between a warp's stage and the ones it writes; a warp whose next stage
+// is in unit y has written every unit below y - kLag, so the MMA of unit y or
+// an earlier one finds its accumulator read
+constexpr int kLag = 4;
+static_assert(kLag < kAccBufs, "the MMA warp waits for accumulators that every warp has passed");
 
-// Per-mode layout.  Split-bf16 (fp32-level accuracy) keeps hi and lo images
-// of both operands: A = hi(B rows) | lo(B rows), values = hi | lo, and
-// issues three MMAs per step (hi*hi + hi*lo + lo*hi); its accumulator is
-// drained into the epilogue's fp32 registers every kGroup steps, which
-// bounds the tensor core's accumulation chain.
-//
-// A bf16 B (kIn16) needs no conversion: the producers copy its rows with
-// cp.async straight into the swizzled A image of the slot (each 16-byte
-// chunk of a row is 8 features, one chunk of the layout), so there is no raw
-// stage and every producer warp keeps two steps in flight in its two slots.
-// Slot s holds the A image(s) at a_off(s) (1024-aligned) and the value
-// image(s) at v_off(s): A images first, then all value images.
-template <int MODE, bool kIn16 = false>
-struct WsCfg {
+// Split-bf16 (fp32-level accuracy) keeps hi and lo images of both operands:
+// A = hi(B rows) | lo(B rows), values = hi | lo, and issues three MMAs per
+// step (hi*hi + hi*lo + lo*hi); its units are 8 k-steps, summed in the
+// epilogue's registers, which bounds the tensor core's accumulation chain.
+template <int MODE, bool kIn16, int kRowF>
+struct TcCfg {
   static constexpr bool kSplit = MODE == STILE_TC_SPLIT_BF16;
-  static constexpr int kSlots = kIn16 ? 3 * kProdWarps : kProdWarps;  // warp w fills slots w, w + 4, ..
-  static constexpr uint32_t kVals = kSplit ? 2 * kBStage : kBStage;   // value image(s) per step
-  static constexpr uint32_t kAImg = kSplit ? 2 * kAStage : kAStage;   // A image(s) per step
-  static constexpr uint32_t kSlotBytes = kSlots * (kAImg + kVals);
-  static constexpr uint32_t kRaw = kIn16 ? 0 : kRawRows + kVals;      // 16 fp32 rows + value image(s)
-  // full / empty barrier per slot, full / empty per accumulator, drain, TMEM address
-  static constexpr uint32_t kBarBytes = (16 * kSlots + 16 * kAccBufs + 16 + 63) / 64 * 64;
-  static constexpr uint32_t kBytes = 1024 + kSlotBytes + kProdWarps * kRaw + kBarBytes;
-  static __device__ __forceinline__ uint32_t a_off(int s) { return (uint32_t)s * kAImg; }
-  static __device__ __forceinline__ uint32_t v_off(int s) { return kSlots * kAImg + (uint32_t)s * kVals; }
-  static constexpr int kCtas = kSplit ? 3 : 4;                        // resident CTAs per SM
-  static constexpr int kGroup = kSplit ? 4 : (1 << 30);               // k-steps per accumulator drain
+  static constexpr int kLanes = kRowF * (kIn16 ? 2 : 4) / 16;  // lanes that cover a gathered row
+  static constexpr int kSpw = kWarp / kLanes;                  // k-steps per stage, rows per load
+  static constexpr uint32_t kVals = kSplit ? 2 * kBStage : kBStage;  // value image(s) of a step
+  // A image of a step: both 64-feature atoms, or only the one that narrow
+  // rows fill (the MMA then reads what follows it as its upper 64 features,
+  // whose accumulator rows nobody reads; kTail keeps that inside the slots)
+  static constexpr uint32_t kAOne = kRowF == 128 ? kAStage : kALbo;
+  static constexpr uint32_t kAImg = kSplit ? 2 * kAOne : kAOne;
+  static constexpr uint32_t kSlot = kSpw * kAImg;
+  static constexpr int kNs = kSlot <= 4096 ? 2 : 1;  // operand slots per warp
+  static constexpr int kNv = kNs + 1;                // value buffers per warp (one is being filled)
+  static constexpr uint32_t kTail = kAStage - kAOne;
+  static constexpr uint32_t kVBuf = kSpw * kVals;
+  static constexpr uint32_t kCBuf = kSpw * 64;       // column ids of a stage; two per warp
+  static constexpr uint32_t kVOff = kTcWarps * kNs * kSlot + kTail;
+  static constexpr uint32_t kCOff = kVOff + kTcWarps * kNv * kVBuf;
+  static constexpr uint32_t kBars = kCOff + kTcWarps * 2 * kCBuf;
+  // full and empty per slot, full and empty per accumulator, drain, TMEM address
+  static constexpr uint32_t kBytes = 1024 + kBars + 16 * kTcWarps * kNs + 16 * kAccBufs + 16;
+  static_assert(kSpw == 1 || kSpw == 2 || kSpw == 4, "a stage is 16 loads");
   static_assert(!(kIn16 && MODE != STILE_TC_BF16), "a bf16 B feeds bf16 MMAs");
+  static_assert(MODE != STILE_TC_FP8 || kSpw == 1, "fp8 converts whole 16-row stages");
+  static_assert(kTcCtas * (kBytes + 1024) <= 228 * 1024, "resident CTAs");
 };
 
-// kFull: every 128-feature slice is complete (N % 128 == 0)
-template <int MODE, bool kFull, bool kIn16>
-__global__ void __launch_bounds__(kWsThreads, WsCfg<MODE, kIn16>::kCtas) spmm_tc_ws_kernel(SpmmArgs p) {
-  using W = WsCfg<MODE, kIn16>;
-  constexpr int kWsSlots = W::kSlots;
+// one warp's bounded wait; the same answer in every lane
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_t polls) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, polls));
+}
+
+// kFull: every feature slice is complete (N % kRowF == 0)
+// kBig: a row of B or C is 4 GB or longer (64-bit row strides)
+template <int MODE, bool kFull, bool kIn16, int kRowF, bool kBig>
+__global__ void __launch_bounds__(kTcThreads, kTcCtas) spmm_tc_kernel(SpmmArgs p) {
+  using W = TcCfg<MODE, kIn16, kRowF>;
+  constexpr int kSpw = W::kSpw, kNs = W::kNs, kNv = W::kNv;
   griddep_launch_dependents();  // the next kernel waits for this grid before using its results
   extern __shared__ uint8_t smem_raw[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t slots = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t ring = slots + W::kSlotBytes;
-  const uint32_t bars = ring + kProdWarps * W::kRaw;
-  // full[kWsSlots], empty[kWsSlots], acc_full[kAccBufs], acc_empty[kAccBufs], drain
-  const uint32_t full0 = bars, empty0 = bars + 8 * kWsSlots;
-  const uint32_t accf0 = bars + 16 * kWsSlots, acce0 = accf0 + 8 * kAccBufs;
-  const uint32_t drain = acce0 + 8 * kAccBufs;
-  const uint32_t tmem_slot = drain + 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  // slot s of warp w: image at base + (kNs w + s) kSlot, barriers full and
+  // empty at bars + 8 (kNs w + s) and kNs kTcWarps further
+  const uint32_t bars = base + W::kBars;
+  const uint32_t full0 = bars, empty0 = bars + 8 * kTcWarps * kNs;
+  const uint32_t accf0 = empty0 + 8 * kTcWarps * kNs, acce0 = accf0 + 8 * kAccBufs;
+  const uint32_t drain = acce0 + 8 * kAccBufs, tmem_slot = drain + 8;
 
-  if (tid == 0) {
-    for (int s = 0; s < kWsSlots; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 1);
-    }
+  // this CTA's first unit, units, first k-step and k-steps
+  const int4 cta = __ldg(p.tc_cta_info + blockIdx.x);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2 * kTcWarps * kNs; ++s) mbar_init(full0 + 8 * s, 1);
     for (int b = 0; b < kAccBufs; ++b) {
       mbar_init(accf0 + 8 * b, 1);
-      mbar_init(acce0 + 8 * b, 4);
+      mbar_init(acce0 + 8 * b, kTcWarps);
     }
     mbar_init(drain, 1);
     fence_mbar_init();
@@ -255,11 +278,11 @@ __global__ void __launch_bounds__(kWsThreads, WsCfg<MODE, kIn16>::kCtas) spmm_tc
   if constexpr (MODE == STILE_TC_FP8) {
     // the A images' upper k halves stay zero (each k-step fills the lower
     // half of a K = 32 operand); made visible to the tensor core's proxy
-    for (int i = tid; i < (int)(kWsSlots * W::kAImg / 16); i += kWsThreads)
-      st_shared_v4(slots + W::a_off(0) + 16 * i, make_uint4(0u, 0u, 0u, 0u));
+    for (int i = threadIdx.x; i < (int)(kTcWarps * kNs * W::kSlot / 16); i += kTcThreads)
+      st_shared_v4(base + 16 * i, make_uint4(0u, 0u, 0u, 0u));
     fence_proxy_async_smem();
   }
-  if (warp == 0) {
+  if (warp == kTcWarps) {
     __syncwarp();
     tmem_alloc(tmem_slot, 16 * kAccBufs);
     tmem_relinquish();
@@ -270,101 +293,135 @@ __global__ void __launch_bounds__(kWsThreads, WsCfg<MODE, kIn16>::kCtas) spmm_tc
   uint32_t tmem;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
 
-  // this CTA's chunks and their contiguous k-steps
-  const int cb = __ldg(p.tc_cta_chunk + blockIdx.x);
-  const int nc = __ldg(p.tc_cta_chunk + blockIdx.x + 1) - cb;
-  const int s_beg = nc > 0 ? __ldg(p.tc_chunk_kbeg + cb) : 0;
-  const int S = nc > 0 ? __ldg(p.tc_chunk_kbeg + cb + nc - 1) + __ldg(p.tc_chunk_nk + cb + nc - 1) - s_beg : 0;
+  const int ub = cta.x, nu = cta.y, s_beg = cta.z, S = cta.w;
   // feature slices of this CTA: blockIdx.y takes [sl0, sl0 + nf) (a wide B
-  // spreads its slices over more CTAs than the chunk schedule has)
+  // spreads its slices over more CTAs than the schedule has)
   const int sl0 = blockIdx.y * p.tc_slice_per;
-  const int nf = min(p.tc_slice_per, p.n_fchunks - sl0);
-  const long T = (long)S * nf;  // this CTA's k-steps over its slices
-  const int n_units = nc * nf;
+  const int nf = nu > 0 ? min(p.tc_slice_per, p.n_fchunks - sl0) : 0;
+  const int Q = (S + kSpw - 1) / kSpw;  // stages per slice
+  const int n_units = nu * nf;
   const int N = p.N;
   const uint32_t polls = p.poll_limit ? p.poll_limit : kDefaultPolls;  // pipeline waits
   bool ok = true;
 
-  if (warp < kProdWarps) {
-    // ---------------- producers ----------------
-    const uint8_t* vals = reinterpret_cast<const uint8_t*>(p.tc_vals) + blockIdx.z * p.tc_vals_head_stride;
-    const uint32_t stage = ring + (uint32_t)warp * W::kRaw;
-    // step g is k-step s_beg + loc of feature slice f0 / 128 (g = f0 / 128 * S + loc)
-    long g = warp;
-    int loc = 0, f0 = 0;
-    if (g < T) {
-      loc = warp % S;
-      f0 = (sl0 + warp / S) * 128;
-    }
-    auto step_cols = [&](long gg, int l) {
-      return (gg < T && lane < 16) ? __ldg(p.tc_cols + (long)(s_beg + l) * 16 + lane) : 0;
-    };
-    // (loc, f0) of this warp's step after the one at (l, ff)
-    auto next_of = [&](int l, int ff, int& ln, int& fn) {
-      ln = l + kProdWarps;
-      fn = ff;
-      while (ln >= S) {
-        ln -= S;
-        fn += 128;
-      }
-    };
-    if constexpr (kIn16) {
-      const uint16_t* B16 = reinterpret_cast<const uint16_t*>(p.B) + blockIdx.z * p.b_head_stride;
-      const int ch = lane & 15, rh = lane >> 4;  // this lane's 16-byte chunk (8 features) and row parity
-      // the step at (l, ff) into `slot`: rows 2j + rh, features ff + 8 ch ..
-      auto issue16 = [&](int cols, int l, int ff, int slot) {
-        const uint32_t sa = slots + W::a_off(slot);
-        const int f = ff + 8 * ch;
-        const uint32_t bytes = kFull ? 16u : ((f + 8 <= N) ? 16u : (f < N ? (uint32_t)(N - f) * 2u : 0u));
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = 2 * j + rh;
-          const int col = __shfl_sync(0xffffffffu, cols, r);
-          const uint16_t* row = B16 + (long)col * p.ldb;
-          cp_async16(sa + a_img_off(8 * ch, r), bytes ? (const void*)(row + f) : (const void*)row, bytes);
-        }
-        cp_async16(slots + W::v_off(slot) + lane * 16, vals + (long)(s_beg + l) * kBStage + lane * 16, 16u);
-        cp_async_commit();
-      };
-      // kD steps of this warp in flight; once the oldest (g) has landed and
-      // the MMA that read its slot last time is done, step g + kD kProdWarps
-      // refills that slot
-      constexpr int kD = kWsSlots / kProdWarps;
-      static_assert(kD >= 1 && kD <= 3, "one to three steps in flight per warp");
-      long gi = g;  // the next step to issue, at (li, fi)
-      int li = loc, fi = f0;
-      for (int d = 0; d < kD && gi < T; ++d) {
-        issue16(step_cols(gi, li), li, fi, (int)(gi % kWsSlots));
-        gi += kProdWarps;
-        next_of(li, fi, li, fi);
-      }
+  if (warp == kTcWarps) {
+    // ---------------- MMA warp ----------------
+    {
+      const bool on = elect_one();
+      // kind::f16 with MN-major A; fp8: e4m3 x e4m3, both operands K-major
+      constexpr uint32_t idesc = (MODE == STILE_TC_F16)   ? make_idesc(0, 0, 1, 0, 128, 16)
+                                 : (MODE == STILE_TC_FP8) ? make_idesc(0, 0, 0, 0, 128, 16)
+                                                          : make_idesc(1, 1, 1, 0, 128, 16);
+      // failure-detection test: nothing arrives on `drain` before the commit
+      // below, so this wait runs out
+      if (p.stall_test && !warp_wait(drain, 0u, polls)) ok = false;
+      int w = 0, round = 0, rv = 0;  // the stage's warp; its how-manieth stage (and that modulo kNv)
+      int l = 0, u1 = 0;             // step in the slice, unit in the slice
+      int n = n_units > 0 ? __ldg(p.tc_unit_meta + ub) & 0xffff : 0;
 #pragma unroll 1
-      for (; g < T; g += kProdWarps) {
-        const int cols_i = step_cols(gi, li);
-        const long pend = (gi - g) / kProdWarps;  // this warp's steps in flight, g the oldest
-        if (pend >= 3) cp_async_wait<2>();
-        else if (pend == 2) cp_async_wait<1>();
-        else cp_async_wait<0>();
-        fence_proxy_async_smem();
-        __syncwarp();
-        const int slot = (int)(g % kWsSlots);
-        if (lane == 0) mbar_arrive(full0 + 8 * slot);
-        if (gi < T) {
-          const uint32_t par = (uint32_t)(g / kWsSlots) & 1u;
-          bool got = true;
-          if (lane == 0) got = mbar_wait_bounded(empty0 + 8 * slot, par, polls);
-          if (!__shfl_sync(0xffffffffu, got, 0)) {
+      for (int t = 0; t < n_units && ok; ++t) {
+        const int b = t % kAccBufs;
+        u1 = u1 + 1 < nu ? u1 + 1 : 0;
+        const int n1 = __ldg(p.tc_unit_meta + ub + u1) & 0xffff;
+        if (t >= kAccBufs && !warp_wait(acce0 + 8 * b, (uint32_t)(t / kAccBufs - 1) & 1u, polls)) {
+          ok = false;
+          break;
+        }
+        const uint32_t d = tmem + (uint32_t)(16 * b);
+#pragma unroll 1
+        for (int s = 0; s < n; ++s) {
+          const int j = l % kSpw;
+          const int slot = kNs * w + (kNs == 2 ? round & 1 : 0);
+          if (j == 0 && !warp_wait(full0 + 8 * slot, (uint32_t)(round / kNs) & 1u, polls)) {
             ok = false;
             break;
           }
-          if (lane != 0) mbar_wait_bounded(empty0 + 8 * slot, par, polls);  // completed: returns at once
-          issue16(cols_i, li, fi, slot);
-          gi += kProdWarps;
-          next_of(li, fi, li, fi);
+          tc_fence_after();
+          const uint32_t sa = base + slot * W::kSlot + j * W::kAImg;
+          const uint32_t sv = base + W::kVOff + (kNv * w + rv) * W::kVBuf + j * W::kVals;
+          if constexpr (MODE == STILE_TC_FP8) {
+            umma_f8_if(on, d, smem_desc(sa, kF8Lbo, kF8Sbo, kSwizzleNone), smem_desc(sv, kF8Lbo, kF8Sbo, kSwizzleNone),
+                    idesc, s > 0 ? 1u : 0u);
+          } else {
+            const uint64_t a_hi = smem_desc(sa, kALbo, kASbo, kSwizzle128B);
+            const uint64_t v_hi = smem_desc(sv, kBLbo, kBSbo, kSwizzleNone);
+            umma_f16_if(on, d, a_hi, v_hi, idesc, s > 0 ? 1u : 0u);
+            if constexpr (W::kSplit) {
+              umma_f16_if(on, d, a_hi, smem_desc(sv + kBStage, kBLbo, kBSbo, kSwizzleNone), idesc, 1u);
+              umma_f16_if(on, d, smem_desc(sa + W::kAOne, kALbo, kASbo, kSwizzle128B), v_hi, idesc, 1u);
+            }
+          }
+          ++l;
+          if (j == kSpw - 1 || l == S) {  // the stage's last k-step
+            umma_commit_if(on, empty0 + 8 * slot);
+            if (++w == kTcWarps) {
+              w = 0;
+              ++round;
+              rv = rv + 1 < kNv ? rv + 1 : 0;
+            }
+          }
+          if (l == S) l = 0;
         }
+        if (ok) umma_commit_if(on, accf0 + 8 * b);
+        n = n1;
       }
-      cp_async_wait<0>();
-    } else {
+      // every MMA this thread issued has completed before TMEM is freed
+      umma_commit_if(on, drain);
+      if (!warp_wait(drain, 0u, kDefaultPolls)) ok = false;
+      if (!ok && lane == 0) atomicOr(p.err_flag, 1);
+    }
+    __syncwarp();
+    griddep_wait();
+  } else {
+    // ---------------- gathering warps ----------------
+    // lane -> k-step rsub of the stage, features fl .. of the slice
+    using T = typename std::conditional<kIn16, uint16_t, float>::type;
+    const int rsub = lane / W::kLanes, fl = (lane % W::kLanes) * (kIn16 ? 8 : 4);
+    // row strides in bytes (one 32 x 32 + 64 bit multiply-add a row)
+    using Stride = typename std::conditional<kBig, unsigned long long, unsigned>::type;
+    const Stride ldb = (Stride)(p.ldb * (long)sizeof(T)), ldc = (Stride)(p.ldc * 4);
+    auto at = [](const char* from, Stride ld, int row) {
+      return kBig ? from + (unsigned long long)row * ld : from + (unsigned long long)(unsigned)row * (unsigned)ld;
+    };
+    const char* Bl = reinterpret_cast<const char*>(reinterpret_cast<const T*>(p.B) + blockIdx.z * p.b_head_stride + fl);
+    const uint32_t cbuf = base + W::kCOff + warp * 2 * W::kCBuf;
+    const uint32_t vbuf = base + W::kVOff + warp * kNv * W::kVBuf;
+    // column ids of stage q into buffer b (past the slice's k-steps: column
+    // 0, a valid row that no MMA reads)
+    const int* my_cols = p.tc_cols + (long)s_beg * 16 + lane * 4;
+    auto copy_cols = [&](int b, int q) {
+      if (lane < 4 * kSpw) {
+        const bool in = kSpw == 1 || q * kSpw + (lane >> 2) < S;
+        cp_async16(cbuf + b * W::kCBuf + lane * 16, in ? my_cols + (long)q * kSpw * 16 : p.tc_cols, in ? 16u : 0u);
+      }
+    };
+    uint4 v[16];  // row i of k-step rsub
+    // loads the rows of the stage whose ids are in buffer b; from: this
+    // lane's features of the slice in row 0
+    auto load_rows = [&](int b, const char* from, bool live) {
+      int c[16];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint4 x = ld_shared_v4(cbuf + b * W::kCBuf + rsub * 64 + 16 * j);
+        c[4 * j] = (int)x.x;
+        c[4 * j + 1] = (int)x.y;
+        c[4 * j + 2] = (int)x.z;
+        c[4 * j + 3] = (int)x.w;
+      }
+      // features past N inside the last 16 bytes are the row's padding: they
+      // only reach accumulator rows that are never stored
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = (kFull || live) ? ldg_u4(at(from, ldb, c[i])) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    const uint8_t* my_vals = reinterpret_cast<const uint8_t*>(p.tc_vals) + blockIdx.z * p.tc_vals_head_stride +
+                             (long)s_beg * W::kVals + lane * 16;
+    auto copy_vals = [&](uint32_t to, int q) {
+      const uint8_t* src = my_vals + (long)q * W::kVBuf;
+#pragma unroll
+      for (int c = 0; c < (int)(W::kVBuf / 512); ++c)
+        if (kSpw == 1 || q * kSpw + c * 512 / (int)W::kVals < S)
+          cp_async16(to + lane * 16 + c * 512, src + c * 512, 16u);
+    };
     // fp8: B's e4m3 scale comes from the run's amax pass, which finished
     // before this kernel started (an ordinary launch never lets a dependent
     // start early)
@@ -373,212 +430,205 @@ __global__ void __launch_bounds__(kWsThreads, WsCfg<MODE, kIn16>::kCtas) spmm_tc
       const float amax = __uint_as_float(*p.tc_xamax);
       xinv = amax > 0.f ? kE4m3Max / amax : 0.f;
     }
-    auto issue = [&](int cols, int l, int ff) {
-      const int f = ff + 4 * lane;
-      const uint32_t bytes = kFull ? 16u : ((f + 4 <= N) ? 16u : (f < N ? (uint32_t)(N - f) * 4u : 0u));
-#pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        const int col = __shfl_sync(0xffffffffu, cols, r);
-        const float* row = p.B + blockIdx.z * p.b_head_stride + (long)col * p.ldb;
-        cp_async16(stage + r * 512 + lane * 16, bytes ? (const void*)(row + f) : (const void*)row, bytes);
-      }
-#pragma unroll
-      for (int c = lane; c < (int)(W::kVals / 16); c += 32)
-        cp_async16(stage + kRawRows + c * 16, vals + (long)(s_beg + l) * W::kVals + c * 16, 16u);
-      cp_async_commit();
-    };
-    if (g < T) issue(step_cols(g, loc), loc, f0);
+
+    // ---- epilogue: the next unit to write, its slice, its meta and output
+    // rows (those of the one after it are loaded while it is written)
+    const int quarter = warp & 3;
+    const bool half0 = warp < 4, half1 = warp >= 3;  // rows 0-7, 8-15 of the tile
+    const int* my_rows = p.tc_unit_rows + (long)ub * 16 + (lane & 15);
+    int e = 0, eu = 0, esl = 0;
+    int meta = n_units > 0 ? __ldg(p.tc_unit_meta + ub) : 0, rows = n_units > 0 ? __ldg(my_rows) : -1;
+    bool waited = false;  // griddep_wait done
+    constexpr int kKeep = W::kSplit ? 2 : 1;  // split-bf16 keeps the sums over the units of a chunk
+    float acc[kKeep][8];
+    // writes units up to and without `upto`
+    auto write_units = [&](int upto) {
 #pragma unroll 1
-    for (; g < T; g += kProdWarps) {
-      // this warp's next step and its column ids (used after the convert)
-      const long gn = g + kProdWarps;
-      int locn, f0n;
-      next_of(loc, f0, locn, f0n);
-      const int coln = step_cols(gn, locn);
-      cp_async_wait<0>();
-      const int slot = (int)(g % kWsSlots);
-      if (g >= kWsSlots) {
-        const uint32_t par = (uint32_t)((g - kWsSlots) / kWsSlots) & 1u;
-        bool got = true;
-        if (lane == 0) got = mbar_wait_bounded(empty0 + 8 * slot, par, polls);
-        if (!__shfl_sync(0xffffffffu, got, 0)) {
-          ok = false;
-          break;
+      while (e < upto) {
+        if (!waited) {
+          // launched dependent on the ELL kernel: the gathers and MMAs start
+          // while it drains, the C writes (adds to rows it stores) wait for it
+          griddep_wait();
+          waited = true;
         }
-        if (lane != 0) mbar_wait_bounded(empty0 + 8 * slot, par, polls);  // completed: returns at once
+        const int b = e % kAccBufs;
+        const int eu1 = eu + 1 < nu ? eu + 1 : 0;
+        const int meta1 = __ldg(p.tc_unit_meta + ub + eu1), rows1 = __ldg(my_rows + (long)eu1 * 16);
+        if (!warp_wait(accf0 + 8 * b, (uint32_t)(e / kAccBufs) & 1u, polls)) {
+          ok = false;
+          return;
+        }
+        tc_fence_after();
+        const bool live = 32 * quarter < kRowF;  // narrow rows: the upper quarters' features do not exist
+        const int f = (sl0 + esl) * 128 + 32 * quarter + lane;
+        const char* Cf = reinterpret_cast<const char*>(p.C + blockIdx.z * p.c_head_stride + f);
+        const bool in = (kFull && kRowF == 128) || f < N;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (!live || !(h ? half1 : half0)) continue;
+          uint32_t r[8];
+          tmem_ld8(tmem + (uint32_t)(16 * b + 8 * h) + ((uint32_t)(32 * quarter) << 16), r);
+          tmem_wait_ld();
+          float(&a)[8] = acc[W::kSplit ? h : 0];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            a[i] = W::kSplit ? ((meta & kUnitFirst) ? 0.f : a[i]) + __uint_as_float(r[i]) : __uint_as_float(r[i]);
+          if (W::kSplit && !(meta & kUnitLast)) continue;
+          if constexpr (MODE == STILE_TC_FP8) {
+            // undo the scales: B's (per tensor) and the tile row's
+            const float sx = __uint_as_float(*p.tc_xamax) / kE4m3Max;
+            const int item = __ldg(p.tc_unit_item + ub + eu);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] *= sx * __ldg(p.tc_row_scale + (long)item * 16 + 8 * h + i);
+          }
+          int row[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) row[i] = __shfl_sync(0xffffffffu, rows, 8 * h + i);
+          if (meta & kUnitAdds) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) red_if(row[i] >= 0 && in, const_cast<char*>(at(Cf, ldc, row[i])), a[i]);
+          } else {
+            // C is not read again: evict first
+#pragma unroll
+            for (int i = 0; i < 8; ++i) st_if(row[i] >= 0 && in, const_cast<char*>(at(Cf, ldc, row[i])), a[i]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acce0 + 8 * b);
+        ++e;
+        eu = eu1;
+        if (eu == 0) ++esl;
+        meta = meta1;
+        rows = rows1;
       }
-      const uint32_t sa = slots + W::a_off(slot);
+    };
+
+    // stage cursors: (sl, q) the stage in registers, (sl1, q1) the next one
+    auto advance = [&](int& sl, int& q) {
+      q += kTcWarps;
+      while (q >= Q) {
+        q -= Q;
+        ++sl;
+      }
+    };
+    const int* my_unit = p.tc_step_unit + s_beg;  // unit (in the slice) of a k-step
+    int sl = nf, q = warp;
+    if (n_units > 0) {
+      sl = 0;
+      while (q >= Q) {
+        q -= Q;
+        ++sl;
+      }
+    }
+    int sl1 = sl, q1 = q, unit = 0, vb = 0, done = 0;
+    if (sl < nf) {
+      copy_cols(0, q);
+      cp_async_commit();
+      advance(sl1, q1);
+      unit = sl * nu + __ldg(my_unit + q * kSpw);
+      cp_async_wait<0>();
+      __syncwarp();
+      copy_vals(vbuf, q);
+      if (sl1 < nf) copy_cols(1, q1);
+      cp_async_commit();
+      load_rows(0, Bl + (sl0 + sl) * 128 * (long)sizeof(T), (sl0 + sl) * 128 + fl < N);
+    }
+    const uint32_t a0 = base + kNs * warp * W::kSlot + (uint32_t)rsub * W::kAImg + a_img_off(fl, 0);
+#pragma unroll 1
+    for (;;) {
+      // write the units well behind this warp's next stage (all of them after
+      // its last one) while the stage's rows arrive
+      write_units(sl < nf ? unit - kLag : n_units);
+      if (!ok || sl >= nf) break;
+      cp_async_wait<0>();
+      __syncwarp();  // this stage's values and the next one's column ids are there
+      // the MMAs of the slot's last stage have read it and its values
+      const int slot = kNs * warp + (kNs == 2 ? done & 1 : 0);
+      if (done >= kNs && !warp_wait(empty0 + 8 * slot, (uint32_t)(done / kNs - 1) & 1u, polls)) {
+        ok = false;
+        break;
+      }
+      const bool more = sl1 < nf;
+      int sl2 = sl1, q2 = q1, unit1 = 0;
+      vb = vb + 1 < kNv ? vb + 1 : 0;  // the next stage's value buffer
+      if (more) {
+        unit1 = __ldg(my_unit + q1 * kSpw);
+        copy_vals(vbuf + vb * W::kVBuf, q1);
+        advance(sl2, q2);
+        if (sl2 < nf) copy_cols(done & 1, q2);
+      }
+      cp_async_commit();
+      const uint32_t to0 = a0 + (kNs == 2 ? (done & 1) * W::kSlot : 0u);
       if constexpr (MODE == STILE_TC_FP8) {
-        // this lane's 4 features x the step's 16 rows -> four K-major
-        // 16-byte rows of the A image (feature m: the e4m3 bytes of x / s_x
-        // for k = 0..15), core matrices of 8 features x 16 bytes
+        // this lane's 4 features x the step's 16 rows -> four K-major 16-byte
+        // rows of the A image (feature m: the e4m3 bytes of x / s_x for
+        // k = 0..15), core matrices of 8 features x 16 bytes
         uint32_t wd[4][4];
 #pragma unroll
         for (int r = 0; r < 16; r += 2) {
-          const uint4 ra = ld_shared_v4(stage + r * 512 + lane * 16);
-          const uint4 rb = ld_shared_v4(stage + (r + 1) * 512 + lane * 16);
-          const uint32_t ua[4] = {ra.x, ra.y, ra.z, ra.w}, ub[4] = {rb.x, rb.y, rb.z, rb.w};
+          const uint32_t ua[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
+          const uint32_t ub4[4] = {v[r + 1].x, v[r + 1].y, v[r + 1].z, v[r + 1].w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const uint32_t h = pack_e4m3x2(__uint_as_float(ua[j]) * xinv, __uint_as_float(ub[j]) * xinv);
+            const uint32_t h = pack_e4m3x2(__uint_as_float(ua[j]) * xinv, __uint_as_float(ub4[j]) * xinv);
             if ((r & 2) == 0) wd[j][r >> 2] = h; else wd[j][r >> 2] |= h << 16;
           }
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int m = 4 * lane + j;
-          st_shared_v4(sa + (uint32_t)((m >> 3) * kF8Sbo + (m & 7) * 16),
+          st_shared_v4(base + slot * W::kSlot + (uint32_t)((m >> 3) * kF8Sbo + (m & 7) * 16),
                        make_uint4(wd[j][0], wd[j][1], wd[j][2], wd[j][3]));
         }
-      }
+      } else {
 #pragma unroll
-      for (int r = 0; r < (MODE == STILE_TC_FP8 ? 0 : 16); ++r) {
-        const uint4 raw = ld_shared_v4(stage + r * 512 + lane * 16);
-        const float4 v = make_float4(__uint_as_float(raw.x), __uint_as_float(raw.y), __uint_as_float(raw.z),
-                                     __uint_as_float(raw.w));
-        const uint32_t o = a_img_off(4 * lane, r);
-        if (MODE == STILE_TC_F16) {
-          st_shared_v2(sa + o, pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
-        } else {
-          const uint32_t h01 = pack_bf16x2(v.x, v.y), h23 = pack_bf16x2(v.z, v.w);
-          st_shared_v2(sa + o, h01, h23);
-          if (W::kSplit) {
-            // lo = v - float(hi): exact in fp32, then rounded to bf16
-            const float4 hf = make_float4(__uint_as_float(h01 << 16), __uint_as_float(h01 & 0xffff0000u),
-                                          __uint_as_float(h23 << 16), __uint_as_float(h23 & 0xffff0000u));
-            st_shared_v2(sa + kAStage + o, pack_bf16x2(v.x - hf.x, v.y - hf.y), pack_bf16x2(v.z - hf.z, v.w - hf.w));
+        for (int i = 0; i < 16; ++i) {
+          // the swizzle XORs the row's low bits into the 16-byte chunk; what
+          // else a row adds to the address is a constant
+          const uint32_t to = (to0 ^ (uint32_t)((i & 7) << 4)) + (uint32_t)((i >> 3) * kASbo + (i & 7) * 128);
+          if constexpr (kIn16) {
+            st_shared_v4(to, v[i]);
+          } else {
+            const float4 x = make_float4(__uint_as_float(v[i].x), __uint_as_float(v[i].y), __uint_as_float(v[i].z),
+                                         __uint_as_float(v[i].w));
+            if constexpr (MODE == STILE_TC_F16) {
+              st_shared_v2(to, pack_f16x2(x.x, x.y), pack_f16x2(x.z, x.w));
+            } else {
+              const uint32_t h01 = pack_bf16x2(x.x, x.y), h23 = pack_bf16x2(x.z, x.w);
+              st_shared_v2(to, h01, h23);
+              if constexpr (W::kSplit) {
+                // lo = x - float(hi): exact in fp32, then rounded to bf16
+                st_shared_v2(to + W::kAOne,
+                             pack_bf16x2(x.x - __uint_as_float(h01 << 16), x.y - __uint_as_float(h01 & 0xffff0000u)),
+                             pack_bf16x2(x.z - __uint_as_float(h23 << 16), x.w - __uint_as_float(h23 & 0xffff0000u)));
+              }
+            }
           }
         }
       }
-#pragma unroll
-      for (int c = lane; c < (int)(W::kVals / 16); c += 32)
-        st_shared_v4(slots + W::v_off(slot) + c * 16, ld_shared_v4(stage + kRawRows + c * 16));
+      if (more) {
+        const char* from = Bl + (sl0 + sl1) * 128 * (long)sizeof(T);
+        load_rows((done + 1) & 1, from, (sl0 + sl1) * 128 + fl < N);
+      }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(full0 + 8 * slot);
-      if (gn < T) issue(coln, locn, f0n);
-      loc = locn;
-      f0 = f0n;
+      ++done;
+      unit = sl1 * nu + unit1;
+      sl = sl1;
+      q = q1;
+      sl1 = sl2;
+      q1 = q2;
     }
     cp_async_wait<0>();
-    }
-  } else if (warp == kProdWarps) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      // fp8: e4m3 x e4m3, both operands K-major
-      const uint32_t idesc = (MODE == STILE_TC_F16)   ? make_idesc(0, 0, 1, 0, 128, 16)
-                             : (MODE == STILE_TC_FP8) ? make_idesc(0, 0, 0, 0, 128, 16)
-                                                      : make_idesc(1, 1, 1, 0, 128, 16);
-      long g = 0;
-      int u = 0;  // accumulation groups issued so far (accumulator u % kAccBufs)
-      // failure-detection test: nothing arrives on `drain` before the
-      // commit below, so this wait runs out
-      if (p.stall_test && !mbar_wait_bounded(drain, 0u, polls)) ok = false;
-#pragma unroll 1
-      for (int t = 0; t < n_units && ok; ++t) {
-        const int n = __ldg(p.tc_chunk_nk + cb + t % nc);
-#pragma unroll 1
-        for (int s0 = 0; s0 < n && ok; s0 += W::kGroup, ++u) {
-          const int b = u % kAccBufs;
-          if (u >= kAccBufs && !mbar_wait_bounded(acce0 + 8 * b, (uint32_t)((u - kAccBufs) / kAccBufs) & 1u, polls)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t d = tmem + (uint32_t)(16 * b);
-          const int s1 = min(n, s0 + W::kGroup);
-#pragma unroll 1
-          for (int s = s0; s < s1; ++s, ++g) {
-            const int slot = (int)(g % kWsSlots);
-            if (!mbar_wait_bounded(full0 + 8 * slot, (uint32_t)(g / kWsSlots) & 1u, polls)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t sa = slots + W::a_off(slot), sv = slots + W::v_off(slot);
-            const uint64_t a_hi = smem_desc(sa, kALbo, kASbo, kSwizzle128B);
-            const uint64_t v_hi = smem_desc(sv, kBLbo, kBSbo, kSwizzleNone);
-            if constexpr (MODE == STILE_TC_FP8)
-              umma_f8(d, smem_desc(sa, kF8Lbo, kF8Sbo, kSwizzleNone), smem_desc(sv, kF8Lbo, kF8Sbo, kSwizzleNone),
-                      idesc, s > s0 ? 1u : 0u);
-            else
-              umma_f16(d, a_hi, v_hi, idesc, s > s0 ? 1u : 0u);
-            if (W::kSplit) {
-              umma_f16(d, a_hi, smem_desc(sv + kBStage, kBLbo, kBSbo, kSwizzleNone), idesc, 1u);
-              umma_f16(d, smem_desc(sa + kAStage, kALbo, kASbo, kSwizzle128B), v_hi, idesc, 1u);
-            }
-            umma_commit(empty0 + 8 * slot);
-          }
-          if (ok) umma_commit(accf0 + 8 * b);
-        }
-      }
-      // every MMA this thread issued has completed before TMEM is freed
-      umma_commit(drain);
-      if (!mbar_wait_bounded(drain, 0u)) ok = false;
-    }
-    __syncwarp();
-  } else {
-    // ---------------- epilogue ----------------
-    // launched dependent on the ELL kernel: the producers and the MMA start
-    // while it drains, the C writes (adds to rows it stores) wait for it
-    griddep_wait();
-    const int quarter = warp & 3;
-    int u = 0;  // accumulation groups consumed so far
-#pragma unroll 1
-    for (int t = 0; t < n_units && ok; ++t) {
-      const int n = __ldg(p.tc_chunk_nk + cb + t % nc);
-      float acc[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-#pragma unroll 1
-      for (int s0 = 0; s0 < n; s0 += W::kGroup, ++u) {
-        const int b = u % kAccBufs;
-        const uint32_t par = (uint32_t)(u / kAccBufs) & 1u;
-        bool got = true;
-        if (lane == 0) got = mbar_wait_bounded(accf0 + 8 * b, par, polls);
-        if (!__shfl_sync(0xffffffffu, got, 0)) {
-          ok = false;
-          break;
-        }
-        if (lane != 0) mbar_wait_bounded(accf0 + 8 * b, par, polls);  // completed: returns at once
-        tc_fence_after();
-        uint32_t r[16];
-        tmem_ld16(tmem + (uint32_t)(16 * b) + ((uint32_t)(32 * quarter) << 16), r);
-        tmem_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acce0 + 8 * b);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) acc[i] += __uint_as_float(r[i]);
-      }
-      if (!ok) break;
-      const int c = cb + t % nc;
-      const int f = (sl0 + t / nc) * 128 + 32 * quarter + lane;
-      if (kFull || f < N) {
-        const int item = __ldg(p.tc_chunk_item + c);
-        const bool atomic = (__ldg(p.tc_chunk_flags + c) & 1) != 0;
-        const int* orows = p.tc_out_rows + (long)item * 16;
-        if constexpr (MODE == STILE_TC_FP8) {
-          // undo the scales: B's (per tensor) and the tile row's
-          const float sx = __uint_as_float(*p.tc_xamax) / kE4m3Max;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) acc[i] *= sx * __ldg(p.tc_row_scale + (long)item * 16 + i);
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int row = __ldg(orows + i);
-          if (row < 0) continue;
-          float* dst = p.C + blockIdx.z * p.c_head_stride + (long)row * p.ldc + f;
-          if (atomic) atomicAdd(dst, acc[i]); else __stcs(dst, acc[i]);  // C is not read again: evict first
-        }
-      }
-    }
+    if (!waited) griddep_wait();
+    if (!ok && lane == 0) atomicOr(p.err_flag, 1);
   }
-  if (!ok) atomicOr(p.err_flag, 1);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) tmem_dealloc(tmem, 16 * kAccBufs);
+  if (warp == kTcWarps) tmem_dealloc(tmem, 16 * kAccBufs);
 }
 
 // ELL tiles as a stream of live entries in row order: records {column,
@@ -1120,20 +1170,38 @@ static cudaError_t resident_ctas(K kernel, int threads, size_t smem, int* sms, i
   return cudaSuccess;
 }
 
-template <int MODE, bool kFull, bool kIn16 = false>
-static cudaError_t launch_ws_t(const SpmmArgs& p, cudaStream_t st) {
-  auto k = spmm_tc_ws_kernel<MODE, kFull, kIn16>;
-  constexpr uint32_t kWsBytes = WsCfg<MODE, kIn16>::kBytes;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWsBytes);
+template <int MODE, bool kFull, bool kIn16 = false, int kRowF = 128, bool kBig = false>
+static cudaError_t launch_tc_t(const SpmmArgs& p, cudaStream_t st) {
+  auto k = spmm_tc_kernel<MODE, kFull, kIn16, kRowF, kBig>;
+  constexpr uint32_t kBytes = TcCfg<MODE, kIn16, kRowF>::kBytes;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBytes);
   if (e != cudaSuccess) return e;
-  // shared memory for the resident CTAs; the rest of the unified L1 /
-  // shared storage stays L1
-  e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  // shared memory for the resident CTAs (1 KB reserved each) out of 228 KB;
+  // the rest of the unified L1 / shared storage stays L1
+  constexpr int kCarveout = (int)((kTcCtas * (kBytes + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));
+  e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout > 100 ? 100 : kCarveout);
   if (e != cudaSuccess) return e;
   if (p.tc_n_chunks == 0 || p.tc_grid == 0) return cudaSuccess;
   return launch_dependent(k, dim3(p.tc_grid, (p.n_fchunks + p.tc_slice_per - 1) / p.tc_slice_per, std::max(1, p.heads)),
-                          dim3(kWsThreads),
-                          kWsBytes, st, p);
+                          dim3(kTcThreads), kBytes, st, p);
+}
+
+// The gathered row of a narrow B: the 32 or 64 features that cover it, so
+// that a load takes 4 or 2 rows (N <= 64 in 16 bits: 4).  The split-bf16 tiles
+// start at 64: four steps' hi and lo images would leave room for one CTA.
+template <int MODE, bool kIn16>
+static cudaError_t launch_tc_rows(const SpmmArgs& p, cudaStream_t st) {
+  if (p.ldb * (kIn16 ? 2 : 4) >= (1L << 32) || p.ldc * 4 >= (1L << 32))
+    return launch_tc_t<MODE, false, kIn16, 128, true>(p, st);
+  if constexpr (!kIn16 && (MODE == STILE_TC_BF16 || MODE == STILE_TC_F16)) {
+    if (p.N == 32) return launch_tc_t<MODE, true, false, 32>(p, st);
+    if (p.N < 32) return launch_tc_t<MODE, false, false, 32>(p, st);
+  }
+  if constexpr (MODE != STILE_TC_FP8) {
+    if (p.N == 64) return launch_tc_t<MODE, true, kIn16, 64>(p, st);
+    if (p.N < 64) return launch_tc_t<MODE, false, kIn16, 64>(p, st);
+  }
+  return p.N % 128 == 0 ? launch_tc_t<MODE, true, kIn16>(p, st) : launch_tc_t<MODE, false, kIn16>(p, st);
 }
 
 // resident CTAs of the tensor-core kernel on the current device, computed
@@ -1152,14 +1220,14 @@ int tc_persistent_ctas(int mode) {
   int sms = 0, per_sm = 0;
   const cudaError_t e =
       mode == STILE_TC_SPLIT_BF16
-          ? resident_ctas(spmm_tc_ws_kernel<STILE_TC_SPLIT_BF16, true, false>, kWsThreads,
-                          WsCfg<STILE_TC_SPLIT_BF16>::kBytes, &sms, &per_sm)
-          : resident_ctas(spmm_tc_ws_kernel<STILE_TC_BF16, true, false>, kWsThreads, WsCfg<STILE_TC_BF16>::kBytes,
-                          &sms, &per_sm);
+          ? resident_ctas(spmm_tc_kernel<STILE_TC_SPLIT_BF16, true, false, 128, false>, kTcThreads,
+                          TcCfg<STILE_TC_SPLIT_BF16, false, 128>::kBytes, &sms, &per_sm)
+          : resident_ctas(spmm_tc_kernel<STILE_TC_BF16, true, false, 128, false>, kTcThreads,
+                          TcCfg<STILE_TC_BF16, false, 128>::kBytes, &sms, &per_sm);
   if (e != cudaSuccess) return 0;
   std::lock_guard<std::mutex> lock(mu);
-  cache[key] = sms * per_sm;
-  return sms * per_sm;
+  cache[key] = sms * std::min(per_sm, kTcCtas);
+  return cache[key];
 }
 
 // Feature slices per CTA of the tensor-core grid.  The chunk schedule
@@ -1182,19 +1250,13 @@ cudaError_t launch_tc(const SpmmArgs& args, cudaStream_t st) {
   p.tc_slice_per = tc_slices_per_cta(p);
   if (p.b_bf16) {
     if (p.tc_mode != STILE_TC_BF16) return cudaErrorNotSupported;
-    return p.N % 128 == 0 ? launch_ws_t<STILE_TC_BF16, true, true>(p, st)
-                          : launch_ws_t<STILE_TC_BF16, false, true>(p, st);
+    return launch_tc_rows<STILE_TC_BF16, true>(p, st);
   }
   switch (p.tc_mode) {
-    case STILE_TC_F16:
-      return p.N % 128 == 0 ? launch_ws_t<STILE_TC_F16, true>(p, st) : launch_ws_t<STILE_TC_F16, false>(p, st);
-    case STILE_TC_FP8:
-      return p.N % 128 == 0 ? launch_ws_t<STILE_TC_FP8, true>(p, st) : launch_ws_t<STILE_TC_FP8, false>(p, st);
-    case STILE_TC_SPLIT_BF16:
-      return p.N % 128 == 0 ? launch_ws_t<STILE_TC_SPLIT_BF16, true>(p, st)
-                            : launch_ws_t<STILE_TC_SPLIT_BF16, false>(p, st);
-    default:
-      return p.N % 128 == 0 ? launch_ws_t<STILE_TC_BF16, true>(p, st) : launch_ws_t<STILE_TC_BF16, false>(p, st);
+    case STILE_TC_F16: return launch_tc_rows<STILE_TC_F16, false>(p, st);
+    case STILE_TC_FP8: return launch_tc_rows<STILE_TC_FP8, false>(p, st);
+    case STILE_TC_SPLIT_BF16: return launch_tc_rows<STILE_TC_SPLIT_BF16, false>(p, st);
+    default: return launch_tc_rows<STILE_TC_BF16, false>(p, st);
   }
 }
 

@@ -29,20 +29,20 @@ struct SpmmArgs {
   int K;          // rows of B
   int n_fchunks;  // ceil(N / 128): tensor-core feature chunks
   int tc_mode;
-  // tensor-core work chunks (items split into runs of <= kChunkSteps k-steps)
+  // tensor-core work chunks (items split into runs of <= kChunkSteps
+  // k-steps), in schedule order
   int tc_n_chunks;
-  const int* tc_chunk_kbeg;   // [tc_n_chunks] first k-step
-  const int* tc_chunk_nk;     // [tc_n_chunks] k-steps
-  // persistent schedule: CTA b owns chunks [tc_cta_chunk[b], tc_cta_chunk[b + 1]),
-  // whose k-steps are contiguous
+  // persistent schedule: {first unit, units, first k-step, k-steps} of every
+  // CTA, whose k-steps are contiguous; a unit is a chunk, or kSplitSteps
+  // k-steps of one in the split-bf16 mode
   int tc_grid;
-  const int* tc_cta_chunk;    // [tc_grid + 1]
-  const int* tc_chunk_item;   // [tc_n_chunks]
-  const int* tc_chunk_flags;  // [tc_n_chunks] bit0: atomic
+  const int4* tc_cta_info;  // [tc_grid]
+  const int* tc_unit_meta;  // [units] k-steps | kUnit flags
+  const int* tc_unit_rows;  // [units * 16] output rows (-1: none)
+  const int* tc_unit_item;  // [units]
+  const int* tc_step_unit;  // [tc_n_ksteps] unit of a k-step, counted within its CTA
   // tensor-core items
   int tc_n_items, tc_n_ksteps;
-  const int* tc_item_kbeg;
-  const int* tc_item_flags;
   const int* tc_out_rows;
   const int* tc_cols;
   const void* tc_vals;
@@ -149,7 +149,10 @@ cudaError_t launch_dvals(const SpmmArgs& p, const float* dY, long lddy, float* d
 cudaError_t launch_tc_dvals(const SpmmArgs& p, const float* X, long ldx, const float* Y, long ldy, float* out, int F,
                             cudaStream_t st);
 constexpr int kTcDvUnit = 8;  // k-steps per unit of the tensor-tile value-gradient kernel
-constexpr int kChunkSteps = 32;
+constexpr int kChunkSteps = 32;  // most k-steps of a chunk
+constexpr int kSplitSteps = 8;   // most k-steps of a unit in the split-bf16 mode
+// unit flags: its rows are added to C; it is a chunk's first, its last unit
+constexpr int kUnitAdds = 1 << 16, kUnitFirst = 1 << 17, kUnitLast = 1 << 18;
 // the tile values of `heads` value sets (vals + h * nnz) into ell_out (+ h *
 // n_ell values) and the tensor-tile images tc_out (+ h * tc_head_bytes);
 // forward_ids: vals are in the forward operator's numbering
