@@ -1094,6 +1094,11 @@ int stile_sddmm_plan_upload(const StileSddmmPlanHost* h, StileSddmmPlan** out) {
       run_ptr.push_back((int32_t)(t + 1));
     }
   }
+  // (an empty mask has no entries to mark)
+  std::vector<bool> in_block((size_t)std::max<int64_t>(h->nnz, 0));
+  for (long e = 0; e < (h->n_blk > 0 ? h->n_blk_nnz : 0); ++e) in_block[h->blk_out[e]] = true;
+  bool disjoint = true;
+  for (long t = 0; t < h->n_1d && disjoint; ++t) disjoint = !in_block[h->remap[t]];
   Arena ar;
   size_t a0 = ar.add(h->mid_idx, (size_t)h->n_1d * 4);
   size_t a1 = ar.add(h->j_idx, (size_t)h->n_1d * 4);
@@ -1140,6 +1145,7 @@ int stile_sddmm_plan_upload(const StileSddmmPlanHost* h, StileSddmmPlan** out) {
   a.n_runs = (int)run_row.size();
   a.run_ptr = P(a8);
   a.run_row = P(a9);
+  a.disjoint = disjoint ? 1 : 0;
   plan->err_flag = (int*)(base + ar.offs[a10]);
   a.err_flag = plan->err_flag;
   e = cudaMemset(plan->err_flag, 0, 16);

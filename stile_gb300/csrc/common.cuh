@@ -432,6 +432,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return d;
 }
 
+// 16-byte chunk q of row `row` of a K-major operand image with the 128-byte
+// swizzle (128-byte rows, 8-row atoms 1 KB apart)
+__device__ __forceinline__ uint32_t sw128_off(int row, int q) {
+  return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((q ^ (row & 7)) << 4));
+}
+
 // Instruction descriptor for kind::f16 / kind::tf32 / kind::f8f6f4 with fp32
 // accumulate.  a_fmt/b_fmt: kind::f16 -> 0 = f16, 1 = bf16; kind::tf32 -> 2;
 // kind::f8f6f4 -> 0 = e4m3.

@@ -413,21 +413,26 @@ cudaError_t launch_sddmm_runs(int n_groups, const int* gptr, const int* grow, co
 //   D[16 j + n][16 j + m] = <X[blk_i[j][m]], Y[blk_j[j][n]]>
 // on the 8 diagonal 16x16 sub-blocks (the off-diagonal ones are products
 // nobody asked for; the tensor pipe has time to spare).  Per 64-feature
-// chunk every thread gathers one Y row and one X row, converts them to bf16
-// (fp32 inputs: hi = bf16(x) and lo = bf16(x - hi), three MMAs per K-slice,
-// hi.hi + hi.lo + lo.hi), stores them in the no-swizzle K-major layout
-// (core matrices of 8 rows x 16 B, k halves 128 B apart, 8-row groups 256 B
-// apart, one 4 KB slice per 16 features), and one thread issues the MMAs
-// into a 128-column TMEM accumulator.  The epilogue reads each warp's 32 Y
-// rows from TMEM, stages the diagonal blocks in shared memory and writes
-// only the blocks' live entries (indicesDense).  The wait for the MMAs is
+// chunk every 16-lane group (8-lane for bf16 operands) gathers its share of
+// the 256 rows, 16 loads in flight per lane, converts them to bf16 (fp32
+// inputs: hi = bf16(x) and lo = bf16(x - hi), three MMAs per K-slice,
+// hi.hi + hi.lo + lo.hi), stores them with the 128-byte swizzle (128-byte
+// rows of 64 features, the 16-byte chunk q of row m at q ^ (m % 8), 8-row
+// atoms 1 KB apart: a group writes whole rows, no bank conflicts), and one
+// thread issues the MMAs into a 128-column TMEM accumulator.  The epilogue
+// reads each warp's 32 Y rows from TMEM, stages the diagonal blocks in shared
+// memory and writes only the blocks' live entries (indicesDense), 4 entries of
+// the unit's contiguous list in flight per thread.  The wait for the MMAs is
 // bounded; a wait that runs out sets the error flag and skips the unit's
 // output.
+// Bound by latency (a mask gives each CTA a unit or two): one thread per row
+// walking its 64 features, and the blocks' entry lists walked one after
+// another, took 17 us for the 1,703 blocks of a 100,000-row mask at F = 64.
 constexpr int kBlkUnit = 8;                      // blocks per unit
 constexpr int kBlkFc = 64;                       // features per chunk: 4 K-slices of 16
-constexpr uint32_t kBlkSlice = 4096;             // one K = 16 slice of 128 bf16 rows
-constexpr uint32_t kBlkImg = 4 * kBlkSlice;      // 64 features of 128 rows
+constexpr uint32_t kBlkImg = 128 * 128;          // 64 bf16 features of 128 rows
 constexpr int kBlkDPad = 17;                     // staged D rows (floats), padded against bank conflicts
+constexpr int kBlkThreads = 256;
 
 template <bool kB16>
 struct BlkCfg {
@@ -436,21 +441,20 @@ struct BlkCfg {
   static constexpr uint32_t kBytes = 1024 + kImgs * kBlkImg + kDBytes + 64;
 };
 
-// 16 bytes of 8 bf16 features at element (row, k = 8 q) of a 128-row
-// K-major image (slice q / 2, k half q % 2)
-__device__ __forceinline__ uint32_t blk_off(int row, int q) {
-  return (uint32_t)((q >> 1) * kBlkSlice + (row >> 3) * 256 + (q & 1) * 128 + (row & 7) * 16);
-}
-
 template <bool kB16>
-__global__ void __launch_bounds__(128) sddmm_block_tc_kernel(SddmmArgs p, int n_units) {
+__global__ void __launch_bounds__(kBlkThreads) sddmm_block_tc_kernel(SddmmArgs p, int n_units, int lazy_wait) {
   using Cfg = BlkCfg<kB16>;
+  // lazy_wait: launched dependent on the 1D kernel of the same call, which
+  // writes other entries; only the end of this grid implies that one's end
+  if (!lazy_wait) griddep_wait();
+  griddep_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t yhi = base, xhi = base + kBlkImg, ylo = base + 2 * kBlkImg, xlo = base + 3 * kBlkImg;
   const uint32_t dst = base + Cfg::kImgs * kBlkImg;
   float* dstage = reinterpret_cast<float*>(smem_raw + (dst - smem_u32(smem_raw)));
   const uint32_t bar = dst + Cfg::kDBytes, tmem_slot = bar + 8;
+  __shared__ int s_ptr[kBlkUnit + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     mbar_init(bar, 1);
@@ -467,6 +471,10 @@ __global__ void __launch_bounds__(128) sddmm_block_tc_kernel(SddmmArgs p, int n_
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
   // kind::f16, bf16 x bf16, M = 128, N = 128, both operands K-major
   constexpr uint32_t idesc = make_idesc(1, 1, 0, 0, 128, 128);
+  constexpr int kLanes = kB16 ? 8 : 16;            // lanes per row (16 bytes each)
+  constexpr int kGroups = kBlkThreads / kLanes;    // rows per load of the block
+  constexpr int kRows = 128 / kGroups;             // rows per lane and side
+  const int grp = tid / kLanes, sl = tid % kLanes;
   const int F = p.F;
   uint32_t phase = 0;
   bool ok = true;
@@ -474,39 +482,45 @@ __global__ void __launch_bounds__(128) sddmm_block_tc_kernel(SddmmArgs p, int n_
   for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
     const int b0 = u * kBlkUnit;
     const int nb = min(kBlkUnit, p.n_blk - b0);
-    const int j = tid >> 4, r = tid & 15;
-    const int yrow = j < nb ? __ldg(p.blk_j + (long)(b0 + j) * 16 + r) : -1;
-    const int xrow = j < nb ? __ldg(p.blk_i + (long)(b0 + j) * 16 + r) : -1;
+    if (tid <= nb) s_ptr[tid] = __ldg(p.blk_indptr + b0 + tid);
+    // this lane's rows: row kGroups i + grp of the unit's 128, per side
+    int row[2][kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int m = kGroups * i + grp;
+      row[0][i] = m < 16 * nb ? __ldg(p.blk_j + (long)b0 * 16 + m) : -1;
+      row[1][i] = m < 16 * nb ? __ldg(p.blk_i + (long)b0 * 16 + m) : -1;
+    }
 #pragma unroll 1
     for (int fc = 0; fc < F; fc += kBlkFc) {
-      // gather and convert: this thread's Y row and X row, 64 features
 #pragma unroll
       for (int side = 0; side < 2; ++side) {
-        const int row = side ? xrow : yrow;
         const uint32_t hi = side ? xhi : yhi, lo = side ? xlo : ylo;
-#pragma unroll 2
-        for (int q = 0; q < kBlkFc / 8; ++q) {
-          const int f = fc + 8 * q;
-          float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-          if (row >= 0) {
-            if constexpr (kB16) {
-              const uint16_t* src = reinterpret_cast<const uint16_t*>(side ? (const void*)p.X : (const void*)p.Y);
-              bf16x8_to_f32(ld_row8_bf16(src + (long)row * (side ? p.ldx : p.ldy), f, F), a, b);
-            } else {
-              const float* src = (side ? p.X : p.Y) + (long)row * (side ? p.ldx : p.ldy);
-              a = ld4_live(src, f, F);
-              b = ld4_live(src, f + 4, F);
-            }
-          }
-          const uint32_t h01 = pack_bf16x2(a.x, a.y), h23 = pack_bf16x2(a.z, a.w);
-          const uint32_t h45 = pack_bf16x2(b.x, b.y), h67 = pack_bf16x2(b.z, b.w);
-          st_shared_v4(hi + blk_off(tid, q), make_uint4(h01, h23, h45, h67));
-          if constexpr (!kB16) {
-            auto lo2 = [](uint32_t h, float x0, float x1) {
-              return pack_bf16x2(x0 - __uint_as_float(h << 16), x1 - __uint_as_float(h & 0xffff0000u));
-            };
-            st_shared_v4(lo + blk_off(tid, q),
-                         make_uint4(lo2(h01, a.x, a.y), lo2(h23, a.z, a.w), lo2(h45, b.x, b.y), lo2(h67, b.z, b.w)));
+        const long ld = side ? p.ldx : p.ldy;
+        if constexpr (kB16) {
+          const uint16_t* src = reinterpret_cast<const uint16_t*>(side ? p.X : p.Y);
+          const int f = fc + 8 * sl;
+          uint4 v[kRows];
+#pragma unroll
+          for (int i = 0; i < kRows; ++i)
+            v[i] = row[side][i] >= 0 ? ld_row8_bf16(src + row[side][i] * ld, f, F) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+          for (int i = 0; i < kRows; ++i) st_shared_v4(hi + sw128_off(kGroups * i + grp, sl), v[i]);
+        } else {
+          const float* src = side ? p.X : p.Y;
+          const int f = fc + 4 * sl;
+          float4 v[kRows];
+#pragma unroll
+          for (int i = 0; i < kRows; ++i)
+            v[i] = row[side][i] >= 0 ? ld4_live(src + row[side][i] * ld, f, F) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int i = 0; i < kRows; ++i) {
+            const uint32_t o = sw128_off(kGroups * i + grp, sl >> 1) + (sl & 1) * 8;
+            const uint32_t h01 = pack_bf16x2(v[i].x, v[i].y), h23 = pack_bf16x2(v[i].z, v[i].w);
+            st_shared_v2(hi + o, h01, h23);
+            st_shared_v2(lo + o,
+                         pack_bf16x2(v[i].x - __uint_as_float(h01 << 16), v[i].y - __uint_as_float(h01 & 0xffff0000u)),
+                         pack_bf16x2(v[i].z - __uint_as_float(h23 << 16), v[i].w - __uint_as_float(h23 & 0xffff0000u)));
           }
         }
       }
@@ -517,12 +531,12 @@ __global__ void __launch_bounds__(128) sddmm_block_tc_kernel(SddmmArgs p, int n_
       if (tid == 0) {
         const int ns = min(4, (F - fc + 15) / 16);
         for (int s = 0; s < ns; ++s) {
-          const uint64_t ah = smem_desc(yhi + s * kBlkSlice, 128, 256, kSwizzleNone);
-          const uint64_t bh = smem_desc(xhi + s * kBlkSlice, 128, 256, kSwizzleNone);
+          const uint64_t ah = smem_desc(yhi + 32 * s, 16, 1024, kSwizzle128B);
+          const uint64_t bh = smem_desc(xhi + 32 * s, 16, 1024, kSwizzle128B);
           umma_f16(tmem, ah, bh, idesc, (fc > 0 || s > 0) ? 1u : 0u);
           if constexpr (!kB16) {
-            umma_f16(tmem, ah, smem_desc(xlo + s * kBlkSlice, 128, 256, kSwizzleNone), idesc, 1u);
-            umma_f16(tmem, smem_desc(ylo + s * kBlkSlice, 128, 256, kSwizzleNone), bh, idesc, 1u);
+            umma_f16(tmem, ah, smem_desc(xlo + 32 * s, 16, 1024, kSwizzle128B), idesc, 1u);
+            umma_f16(tmem, smem_desc(ylo + 32 * s, 16, 1024, kSwizzle128B), bh, idesc, 1u);
           }
         }
         umma_commit(bar);
@@ -538,13 +552,13 @@ __global__ void __launch_bounds__(128) sddmm_block_tc_kernel(SddmmArgs p, int n_
       tc_fence_after();
     }
     if (!ok) break;
-    // epilogue: warp w holds TMEM lanes (Y rows) 32 w .. 32 w + 31, i.e.
+    // epilogue: warp w < 4 holds TMEM lanes (Y rows) 32 w .. 32 w + 31, i.e.
     // blocks 2 w and 2 w + 1, whose X rows are TMEM columns 16 j .. 16 j + 15
-    uint32_t v0[16], v1[16];
-    tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(32 * warp), v0);
-    tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(32 * warp + 16), v1);
-    tmem_wait_ld();
-    {
+    if (warp < 4) {
+      uint32_t v0[16], v1[16];
+      tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(32 * warp), v0);
+      tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(32 * warp + 16), v1);
+      tmem_wait_ld();
       const int jj = tid >> 4, n = tid & 15;
 #pragma unroll
       for (int m = 0; m < 16; ++m)
@@ -552,16 +566,34 @@ __global__ void __launch_bounds__(128) sddmm_block_tc_kernel(SddmmArgs p, int n_
     }
     tc_fence_before();
     __syncthreads();
-    for (int jj = 0; jj < nb; ++jj) {
-      const int e0 = __ldg(p.blk_indptr + b0 + jj), e1 = __ldg(p.blk_indptr + b0 + jj + 1);
-      for (int e = e0 + tid; e < e1; e += 128) {
-        const int pos = __ldg(p.blk_dense_pos + e);
-        const int m = pos / p.bn, n = pos % p.bn;
-        __stcs(p.out + __ldg(p.blk_out + e), dstage[(jj * 16 + n) * kBlkDPad + m]);
+    // the unit's entries are one list: which block an entry belongs to comes
+    // from the blocks' bounds
+    const int e1 = s_ptr[nb];
+    auto block_of = [&](int e) {
+      int jj = 0;
+#pragma unroll
+      for (int b = 1; b < kBlkUnit; ++b) jj += (b < nb && e >= s_ptr[b]) ? 1 : 0;
+      return jj;
+    };
+#pragma unroll 1
+    for (int e = s_ptr[0] + tid; e < e1; e += 4 * kBlkThreads) {
+      int pos[4], to[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = min(e + i * kBlkThreads, e1 - 1);
+        pos[i] = __ldg(p.blk_dense_pos + t);
+        to[i] = __ldg(p.blk_out + t);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = e + i * kBlkThreads;
+        if (t < e1)  // 16 x 16 blocks: position 16 m + n
+          __stcs(p.out + to[i], dstage[(block_of(t) * 16 + (pos[i] & 15)) * kBlkDPad + (pos[i] >> 4)]);
       }
     }
     __syncthreads();
   }
+  if (lazy_wait) griddep_wait();
   if (!ok && tid == 0 && p.err_flag) atomicOr(p.err_flag, 1);
   // every MMA this CTA issued has completed before TMEM is freed
   if (!ok && tid == 0) mbar_wait_bounded(bar, phase ^ 1u);
@@ -571,27 +603,36 @@ __global__ void __launch_bounds__(128) sddmm_block_tc_kernel(SddmmArgs p, int n_
   if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
+static cudaError_t launch_blocks(const SddmmArgs& p, bool lazy_wait, cudaStream_t st) {
+  if (p.n_blk == 0) return cudaSuccess;
+  if (p.bm != 16 || p.bn != 16) return cudaErrorNotSupported;
+  const int n_units = (p.n_blk + kBlkUnit - 1) / kBlkUnit;
+  // at least 56 KB of shared memory per CTA: at most 4 CTAs share an SM,
+  // whose 512 TMEM columns then hold their 128-column accumulators
+  const size_t smem = std::max<size_t>(p.xy_bf16 ? BlkCfg<true>::kBytes : BlkCfg<false>::kBytes, 56 * 1024);
+  auto k = p.xy_bf16 ? sddmm_block_tc_kernel<true> : sddmm_block_tc_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int grid = std::min(n_units, device_sm_count() * (p.xy_bf16 ? 4 : 2));
+  return launch_dependent(k, dim3(grid), dim3(kBlkThreads), smem, st, p, n_units, lazy_wait ? 1 : 0);
+}
+
 cudaError_t launch_sddmm(const SddmmArgs& p, cudaStream_t st) {
-  // block tiles first, then 1D tiles: where both cover a nonzero the 1D
+  // Block tiles first, then 1D tiles: where both cover a nonzero the 1D
   // result is the one kept, as in the reference's host reorder
-  // (order_output_BSDDMM writes the TC results first, then the 1D ones)
-  if (p.n_blk > 0) {
-    if (p.bm != 16 || p.bn != 16) return cudaErrorNotSupported;
-    const int n_units = (p.n_blk + kBlkUnit - 1) / kBlkUnit;
-    // at least 57 KB of shared memory per CTA: at most 4 CTAs share an SM,
-    // whose 512 TMEM columns then hold their 128-column accumulators
-    const size_t smem = std::max<size_t>(p.xy_bf16 ? BlkCfg<true>::kBytes : BlkCfg<false>::kBytes, 57 * 1024);
-    auto k = p.xy_bf16 ? sddmm_block_tc_kernel<true> : sddmm_block_tc_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    const int grid = std::min(n_units, device_sm_count() * (p.xy_bf16 ? 4 : 2));
-    k<<<grid, 128, smem, st>>>(p, n_units);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  // 1D tiles: the flattened entries come in runs of one row (cut at upload)
-  return launch_sddmm_runs(p.n_runs, p.run_ptr, p.run_row, p.j_idx, p.remap, p.X, p.xy_bf16, p.ldx, p.Y, p.xy_bf16,
-                           p.ldy, p.out, p.F, st);
+  // (order_output_BSDDMM writes the TC results first, then the 1D ones).
+  // Where no entry is in both (checked at upload) the order is free: the 1D
+  // kernel goes first and the block kernel's few CTAs start on the SMs that
+  // its last wave leaves.  (The 1D kernel beside the block kernel kept the
+  // SMs at that one's shared-memory size, with less L1: 74 us on the
+  // 100,000-row mask at F = 64, 54 us alone.)
+  cudaError_t e = cudaSuccess;
+  if (!p.disjoint && (e = launch_blocks(p, false, st)) != cudaSuccess) return e;
+  // the flattened entries come in runs of one row (cut at upload)
+  e = launch_sddmm_runs(p.n_runs, p.run_ptr, p.run_row, p.j_idx, p.remap, p.X, p.xy_bf16, p.ldx, p.Y, p.xy_bf16, p.ldy,
+                        p.out, p.F, st);
+  if (e != cudaSuccess || !p.disjoint) return e;
+  return launch_blocks(p, p.n_runs > 0, st);
 }
 
 // Row softmax over a CSR pattern (the sparse-attention step between the

@@ -1424,10 +1424,6 @@ constexpr uint32_t kDvYImg = 16384;  // 128 rows x 64 bf16
 constexpr uint32_t kDvXImg = 2048;   // 16 rows x 64 bf16
 constexpr uint32_t kDvBytes = 1024 + 2 * kDvYImg + 2 * kDvXImg + 64 + 64;
 
-__device__ __forceinline__ uint32_t sw128_off(int row, int q) {
-  return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((q ^ (row & 7)) << 4));
-}
-
 constexpr int kDvThreads = 256;
 
 __global__ void __launch_bounds__(kDvThreads, 3) spmm_tc_dvals_kernel(SpmmArgs p, const float* __restrict__ X, long ldx,

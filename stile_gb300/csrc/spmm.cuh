@@ -184,6 +184,7 @@ struct SddmmArgs {
   const int* blk_indptr;
   const int* blk_dense_pos;
   const int* blk_out;
+  int disjoint;  // no entry is in a 1D and in a block tile
   // device error flag (the block kernel's bounded MMA wait gave up)
   int* err_flag;
 };
