@@ -64,6 +64,18 @@ struct StileSpmmPlan {
   bool ids_set = false;  // set_transpose_ids has run
 };
 
+// Most entries of a run group: kRunGroup, or 32, 16 or 8 where that gives fewer
+// than two groups per warp the device keeps resident (48 per SM).  A group
+// gathers its rows a few at a time, so a small list is bound by its longest
+// group: 430,000 entries at 100 bf16 features took 26 us in groups of 64 with
+// the mean at 20; a large list keeps long groups, which load their row once.
+static int run_group(long entries) {
+  const long warps = 2L * stile::device_sm_count() * 48;
+  int cap = stile::kRunGroup;
+  while (cap > 8 && entries / cap < warps) cap /= 2;
+  return cap;
+}
+
 // default of the tensor tiles' value gradients: the row runs (measured
 // faster on the GCN graph, 40.7 nonzeros per k-step: the tensor-core kernel
 // gathers fewer rows, but each CTA waits for its loads, then its MMAs, per
@@ -442,13 +454,14 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
       }
     }
   const long ndv = (long)dv_id.size();
-  // runs of one row, cut at kRunGroup entries and where the tensor-core
+  // runs of one row, cut at `run_cap` entries and where the tensor-core
   // entries end (the row-run kernel's groups; the tensor-core prefix alone
   // serves the fused backward)
+  const int run_cap = run_group(ndv);
   std::vector<int32_t> dv_gptr{0}, dv_grow;
   int dv_groups_tc = 0;
   for (long t = 0; t < ndv; ++t) {
-    const bool cut = t + 1 == ndv || dv_row[t + 1] != dv_row[t] || t + 1 - dv_gptr.back() == stile::kRunGroup ||
+    const bool cut = t + 1 == ndv || dv_row[t + 1] != dv_row[t] || t + 1 - dv_gptr.back() == run_cap ||
                      t + 1 == n_tc_dv;
     if (t + 1 == n_tc_dv) dv_groups_tc = (int)dv_grow.size() + 1;
     if (cut) {
@@ -1086,10 +1099,11 @@ int stile_sddmm_plan_upload(const StileSddmmPlanHost* h, StileSddmmPlan** out) {
         !in_range(h->blk_out, h->n_blk_nnz, 0, h->nnz))
       return fail(STILE_E_INVALID, "block index out of range");
   }
-  // the 1D entries as runs of one row, cut at stile::kRunGroup entries
+  // the 1D entries as runs of one row, cut at `run_cap` entries
+  const int run_cap = run_group(h->n_1d);
   std::vector<int32_t> run_ptr{0}, run_row;
   for (long t = 0; t < h->n_1d; ++t) {
-    if (t + 1 == h->n_1d || h->mid_idx[t + 1] != h->mid_idx[t] || t + 1 - run_ptr.back() == stile::kRunGroup) {
+    if (t + 1 == h->n_1d || h->mid_idx[t + 1] != h->mid_idx[t] || t + 1 - run_ptr.back() == run_cap) {
       run_row.push_back(h->mid_idx[t]);
       run_ptr.push_back((int32_t)(t + 1));
     }
