@@ -361,6 +361,13 @@ int stile_spmm_plan_set_wait_policy(StileSpmmPlan* plan, int32_t polls, int32_t 
 int stile_debug_umma_probe(const void* a_img, const void* b_img, const uint32_t* desc6,
                            uint32_t idesc, int32_t kind, float* out, int32_t* err, void* stream);
 
+/* Dense operand rows as the kernels read them: `rows` rows of `cols` elements
+ * of 2 or 4 bytes, src_ld elements apart (any stride and alignment of whole
+ * elements), into rows of dst_ld elements (dst_ld * elem_bytes a multiple of
+ * 16, dst 16-byte aligned); the elements past cols become 0. */
+int stile_pad_rows(const void* src, int64_t rows, int32_t cols, int64_t src_ld,
+                   int32_t elem_bytes, void* dst, int64_t dst_ld, void* stream);
+
 /* Copy the last error message of the calling thread into buf. */
 int stile_last_error(char* buf, size_t n);
 

@@ -1041,6 +1041,25 @@ int stile_sddmm_plan_error_flag(StileSddmmPlan* plan, void* stream, int32_t* fla
   return STILE_OK;
 }
 
+int stile_pad_rows(const void* src, int64_t rows, int32_t cols, int64_t src_ld, int32_t elem_bytes, void* dst,
+                   int64_t dst_ld, void* stream) {
+  stile::begin_call();
+  if (rows < 0 || cols < 0) return fail(STILE_E_INVALID, "bad shape");
+  if (elem_bytes != 2 && elem_bytes != 4) return fail(STILE_E_UNSUPPORTED, "elements of 2 or 4 bytes");
+  if (rows == 0 || cols == 0) return STILE_OK;
+  if (!src || !dst) return fail(STILE_E_INVALID, "null argument");
+  if (dst_ld < cols || (dst_ld * elem_bytes) % 16 != 0 || (reinterpret_cast<uintptr_t>(dst) & 15) != 0)
+    return fail(STILE_E_INVALID, "dst: rows of whole 16-byte vectors, 16-byte aligned");
+  if ((reinterpret_cast<uintptr_t>(src) & (elem_bytes - 1)) != 0) return fail(STILE_E_INVALID, "src: misaligned elements");
+  if (rows > (INT64_C(1) << 38) / (dst_ld * elem_bytes / 16))
+    return fail(STILE_E_UNSUPPORTED, "more rows than one launch covers");
+  cudaError_t e = stile::launch_pad_rows(src, (long)rows, cols, src_ld, elem_bytes, dst, dst_ld,
+                                         static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "row padding launch");
+  g_launches++;
+  return STILE_OK;
+}
+
 int stile_csr_row_softmax(int32_t M, const int32_t* indptr, int64_t nnz, const float* x, float* out, float scale,
                           int32_t batch, void* stream) {
   stile::begin_call();

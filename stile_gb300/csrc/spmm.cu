@@ -1065,6 +1065,42 @@ __global__ void amax_kernel(const float* __restrict__ B, long ldb, int K, int N,
   if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(out, __float_as_uint(m));
 }
 
+// Rows of `cols` elements (any row stride, any alignment) into rows of ld
+// elements, zeros past cols: the operand rows of the gathering kernels are
+// 16-byte vectors.  Bound by memory: a thread writes one 16-byte vector; its
+// element loads share sectors with its neighbours' in L1.
+template <typename T>
+__global__ void __launch_bounds__(256) pad_rows_kernel(const T* __restrict__ src, long rows, int cols, long src_ld,
+                                                       uint4* __restrict__ dst, unsigned vecs) {
+  constexpr int kPer = 16 / sizeof(T);
+  const long i = (long)blockIdx.x * 256 + threadIdx.x;
+  const long r = i / vecs;
+  if (r >= rows) return;
+  const int c = (int)(i - r * vecs) * kPer;
+  const T* from = src + r * src_ld + c;
+  union {
+    T e[kPer];
+    uint4 v;
+  } x;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) x.e[k] = c + k < cols ? __ldg(from + k) : T(0);
+  dst[i] = x.v;
+}
+
+cudaError_t launch_pad_rows(const void* src, long rows, int cols, long src_ld, int elem_bytes, void* dst, long dst_ld,
+                            cudaStream_t st) {
+  if (rows <= 0 || cols <= 0) return cudaSuccess;
+  const long vecs = dst_ld * elem_bytes / 16;
+  const unsigned grid = (unsigned)((rows * vecs + 255) / 256);
+  if (elem_bytes == 4)
+    pad_rows_kernel<<<grid, 256, 0, st>>>(static_cast<const unsigned*>(src), rows, cols, src_ld,
+                                          static_cast<uint4*>(dst), (unsigned)vecs);
+  else
+    pad_rows_kernel<<<grid, 256, 0, st>>>(static_cast<const unsigned short*>(src), rows, cols, src_ld,
+                                          static_cast<uint4*>(dst), (unsigned)vecs);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_amax(const float* B, long ldb, int K, int N, unsigned* amax_bits, cudaStream_t st) {
   const long total = (long)K * N;
   if (total == 0) return cudaSuccess;

@@ -162,6 +162,11 @@ cudaError_t launch_pack_values(const SpmmArgs& p, const float* vals, long nnz, i
 // the non-negative floats' bits; *amax_bits starts at 0); an ordinary launch
 cudaError_t launch_amax(const float* B, long ldb, int K, int N, unsigned* amax_bits, cudaStream_t st);
 
+// rows of `cols` elements of 2 or 4 bytes, src_ld elements apart, into rows of
+// dst_ld elements (whole 16-byte vectors), zeros past cols
+cudaError_t launch_pad_rows(const void* src, long rows, int cols, long src_ld, int elem_bytes, void* dst, long dst_ld,
+                            cudaStream_t st);
+
 struct SddmmArgs {
   const float* X;  // fp32, or bf16 bits when xy_bf16 (X and Y alike)
   long ldx;

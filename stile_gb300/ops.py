@@ -36,12 +36,24 @@ def dense_operand(x: torch.Tensor, name="B"):
     ld = x.stride(0)
     ok = x.stride(1) == 1 and ld >= cols and ld % 4 == 0 and x.data_ptr() % 16 == 0
     if not ok:
-        ldp = (cols + 3) // 4 * 4
-        buf = torch.zeros((rows, ldp), dtype=torch.float32, device=x.device)
-        buf[:, :cols] = x
-        x = buf[:, :cols]
-        ld = ldp
+        ld = (cols + 3) // 4 * 4
+        x = _padded_rows(x, ld)
     return x, ld
+
+
+def _padded_rows(x: torch.Tensor, ldp: int) -> torch.Tensor:
+    """x [rows, cols] as a view of a [rows, ldp] buffer whose padding is zero.
+    Rows of contiguous elements go through the padding kernel (one pass over
+    memory), other strides through torch."""
+    rows, cols = x.shape
+    if x.stride(1) != 1 or x.requires_grad or rows * ldp >= 1 << 39:
+        buf = torch.zeros((rows, ldp), dtype=x.dtype, device=x.device)
+        buf[:, :cols] = x
+        return buf[:, :cols]
+    buf = torch.empty((rows, ldp), dtype=x.dtype, device=x.device)
+    _lib.check(_lib.load().stile_pad_rows(x.data_ptr(), rows, cols, x.stride(0), x.element_size(), buf.data_ptr(),
+                                          ldp, _stream()), "stile_pad_rows")
+    return buf[:, :cols]
 
 
 def dense_operand_bf16(x: torch.Tensor, name="B"):
@@ -56,11 +68,8 @@ def dense_operand_bf16(x: torch.Tensor, name="B"):
     ld = x.stride(0)
     ok = x.stride(1) == 1 and ld >= cols and ld % 8 == 0 and x.data_ptr() % 16 == 0
     if not ok:
-        ldp = (cols + 7) // 8 * 8
-        buf = torch.zeros((rows, ldp), dtype=torch.bfloat16, device=x.device)
-        buf[:, :cols] = x
-        x = buf[:, :cols]
-        ld = ldp
+        ld = (cols + 7) // 8 * 8
+        x = _padded_rows(x, ld)
     return x, ld
 
 
