@@ -232,9 +232,9 @@ class SpmmOperator:
     def backward(self, dC: torch.Tensor, B: torch.Tensor, dB: torch.Tensor | None = None):
         """(dB = A^T @ dC, dvals = <dC[row], B[col]> on A's pattern), fp32 dC
         and B: fused (one pass over the transposed plan's row tiles) or
-        separate (transposed product, then the value-gradient pass), each
-        with the tensor-tile nonzeros' gradients on the tensor cores or by
-        row runs, or the plain CSR kernels (path="csr").  With
+        separate (transposed product, then the value-gradient pass), with the
+        tensor-tile nonzeros' gradients by row runs in fp32, or the plain CSR
+        kernels (path="csr").  With
         ``cfg.backward="auto"`` or ``cfg.path="auto"`` the first backward of
         each width times the allowed variants on its operands and keeps the
         fastest."""
@@ -252,45 +252,36 @@ class SpmmOperator:
             _, csrT, sd = self._plain_ops()
             dvals = sd.run(dC, B)
             return csrT.spmm(dC, dB), dvals
-        # "_tc": the tensor-tile nonzeros' gradients on the tensor cores
-        mode = 1 if choice.endswith("_tc") else 2
-        if choice.startswith("fused"):
-            opT.handle.set_dvals_mode(mode)
+        if choice == "fused":
+            opT.handle.set_dvals_mode(2)
             return opT.handle.backward(dC, B, dB)
-        self.handle.set_dvals_mode(mode)
+        self.handle.set_dvals_mode(2)
         dvals = self.handle.dvals(dC, B)
         return opT.handle.run(dC, dB), dvals
 
     def _tune_backward(self, opT, dC, B):
         """The fastest backward variant on these operands (the median of
         three CUDA-event timings after a warm-up call): fused or separate as
-        the config allows, each with the tensor-tile value gradients on the
-        tensor cores ("_tc") or by row runs, and the plain CSR kernels with
-        path="auto"."""
-        def fused(mode):
-            def run():
-                opT.handle.set_dvals_mode(mode)
-                opT.handle.backward(dC, B)
-            return run
+        the config allows, and the plain CSR kernels with path="auto".  The
+        tensor-tile value gradients on the tensor cores (set_dvals_mode(1))
+        are no candidate: their hi + lo products are off by 3e-6 where the
+        fp32 row runs are off by 7e-8, and which of the two a step returned
+        would depend on the timing."""
+        def fused():
+            opT.handle.set_dvals_mode(2)
+            opT.handle.backward(dC, B)
 
-        def separate(mode):
-            def run():
-                self.handle.set_dvals_mode(mode)
-                self.handle.dvals(dC, B)
-                opT.handle.run(dC)
-            return run
+        def separate():
+            self.handle.set_dvals_mode(2)
+            self.handle.dvals(dC, B)
+            opT.handle.run(dC)
 
         def plain():
             _, csrT, sd = self._plain_ops()
             sd.run(dC, B)
             csrT.spmm(dC)
         families = ["fused", "separate"] if self.cfg.backward == "auto" else [self.cfg.backward]
-        cands = {}
-        for fam in families:
-            make = fused if fam == "fused" else separate
-            cands[fam] = make(2)
-            if (opT if fam == "fused" else self).handle.has_tensor_tiles:
-                cands[fam + "_tc"] = make(1)
+        cands = {fam: fused if fam == "fused" else separate for fam in families}
         if self.cfg.path == "auto":
             cands["csr"] = plain
         times = {name: _median_ms(fn) for name, fn in cands.items()}

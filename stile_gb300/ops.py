@@ -16,7 +16,12 @@ def _ptr(a: np.ndarray, ct=ctypes.c_int32):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device, as the address the C entry
+    points take (torch.cuda.current_stream() builds a Stream object: 4 us a
+    call, and a training step makes six)."""
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _require_cuda(t: torch.Tensor, name: str):
@@ -76,7 +81,7 @@ def dense_operand_bf16(x: torch.Tensor, name="B"):
 def new_output(rows, cols, device):
     ldp = (cols + 3) // 4 * 4
     buf = torch.empty((rows, ldp), dtype=torch.float32, device=device)
-    return buf[:, :cols], ldp
+    return (buf if ldp == cols else buf[:, :cols]), ldp
 
 
 def output_operand(out: torch.Tensor | None, rows: int, cols: int, device):
@@ -209,6 +214,7 @@ class DeviceSpmmPlan:
                    "stile_spmm_plan_upload")
         self.handle = handle
         self._dvals_cover_all = _tiles_cover_every_nonzero(dev)
+        self._dvals_mode = 0  # as set_dvals_mode set it last (0: as uploaded)
         # tensor tiles with nonzero ids: their value gradients can run on the
         # tensor cores (stile_spmm_plan_set_dvals_mode)
         self.has_tensor_tiles = len(dev.tc_cols) > 0 and len(dev.tc_nnz_id) > 0
@@ -331,7 +337,10 @@ class DeviceSpmmPlan:
     def set_dvals_mode(self, mode: int):
         """Value gradients of the tensor-tile nonzeros: 0 automatic, 1 on the
         tensor cores, 2 by the row runs (stile_spmm_plan_set_dvals_mode)."""
+        if int(mode) == self._dvals_mode:
+            return
         _lib.check(self.lib.stile_spmm_plan_set_dvals_mode(self.handle, int(mode)), "stile_spmm_plan_set_dvals_mode")
+        self._dvals_mode = int(mode)
 
     def error_flag(self) -> int:
         f = ctypes.c_int32(0)
@@ -361,6 +370,11 @@ class DeviceSddmmPlan:
         _lib.check(self.lib.stile_sddmm_plan_upload(ctypes.byref(h), ctypes.byref(handle)),
                    "stile_sddmm_plan_upload")
         self.handle = handle
+        # every entry is in a tile: a run writes all of its output
+        hit = np.zeros(dev.nnz, dtype=bool)
+        hit[dev.remap] = True
+        hit[dev.blk_out] = True
+        self._cover_all = bool(hit.all())
 
     def error_flag(self) -> int:
         f = ctypes.c_int32(0)
@@ -381,7 +395,8 @@ class DeviceSddmmPlan:
         if X.shape[1] != Y.shape[1]:
             raise ValueError("X and Y must have the same feature count")
         if out is None:
-            out = torch.zeros(self.nnz, dtype=torch.float32, device=X.device)
+            alloc = torch.empty if self._cover_all else torch.zeros
+            out = alloc(self.nnz, dtype=torch.float32, device=X.device)
         fn = self.lib.stile_sddmm_run_bf16 if bf16 else self.lib.stile_sddmm_run
         _lib.check(fn(self.handle, X.data_ptr(), ldx, Y.data_ptr(), ldy, out.data_ptr(), X.shape[1], _stream()),
                    "stile_sddmm_run_bf16" if bf16 else "stile_sddmm_run")
