@@ -8,79 +8,173 @@
 // the scores on the pattern, the row softmax of the sparse transformer
 // (my_3rdparty/Magicube/Magicube1/end2end_eval/sparse_transformer_magicube/
 // src/cuda/softmax_kernel.cu) and the SpMM with the probabilities as values,
-// here in one pass per row: an LPR-lane group holds its query row (8
-// features a lane, as two float4 4 LPR features apart), gathers the K and V rows of two entries at a time,
-// reduces the two scores with a transposing butterfly, broadcasts them, and
-// keeps an online softmax -- running maximum m, running sum l and an output
-// accumulator rescaled by exp(m_old - m_new) whenever the maximum grows --
-// so neither the scores nor the probabilities are written anywhere.
+// here in one pass per row: an LPR-lane group holds its query row (8 features
+// a lane, as two float4 4 LPR features apart), takes the row's entries kU at a
+// time with their K and V rows in flight, and reduces the kU scores with a
+// transposing butterfly, so that each lane holds one entry's score and takes
+// one exponential for it.  An online softmax -- running maximum m, a sum l per
+// entry slot, and an output accumulator rescaled by exp(m_old - m_new) -- keeps
+// the scores and the probabilities out of memory.
+//
+// Bound by instruction issue before and by the L1 data pipe now (a strided
+// mask's neighbouring rows share their columns: two thirds of the loads hit
+// L1, and 3.1 GB of K and V rows pass the pipe): the multiply-adds are paired
+// (fma.rn.f32x2), the column ids come LPR at a time, full rows load without
+// masks and one exponential a batch serves its kU entries.  4096 tokens, 8
+// heads, 64 features, strided mask (766k entries a head): 188 us with pairs of
+// entries and scalar multiply-adds, 152 us now.
 #include "common.cuh"
 #include "spmm.cuh"
 
 namespace stile {
 
-template <int LPR>
-__global__ void __launch_bounds__(256, 4) sparse_attention_kernel(int n_rows, const int* __restrict__ indptr,
-                                                                   const int* __restrict__ indices,
-                                                                   const float* __restrict__ Q,
-                                                                   const float* __restrict__ K,
-                                                                   const float* __restrict__ V, long ldq, long ldk,
-                                                                   long ldv, long q_head, long k_head, long v_head,
-                                                                   float* __restrict__ out, long ldo, long o_head,
-                                                                   int F, int Fv, float scale) {
-  static_assert(LPR >= 2, "two entries per batch");
+struct Feat8 {  // this lane's 8 features of a row: f .. f + 3 and f2 .. f2 + 3
+  f32x2 v[4];
+};
+
+// kMask 0: the row has all 8 LPR features; 1: whole float4 up to n; 2: any n
+// (features past n are zero)
+template <int kMask>
+__device__ __forceinline__ Feat8 load8(const float* row, int f, int f2, int n) {
+  float4 a, b;
+  if constexpr (kMask == 0) {
+    a = ldg4(row + f);
+    b = ldg4(row + f2);
+  } else if constexpr (kMask == 1) {
+    a = ld4_pad(row, f, n);
+    b = ld4_pad(row, f2, n);
+  } else {
+    a = ld4_live(row, f, n);
+    b = ld4_live(row, f2, n);
+  }
+  return {{pack2(a.x, a.y), pack2(a.z, a.w), pack2(b.x, b.y), pack2(b.z, b.w)}};
+}
+
+constexpr int kAttThreads = 128;
+
+template <int LPR, int kMask>
+__global__ void __launch_bounds__(kAttThreads, 5) sparse_attention_kernel(
+    int n_rows, const int* __restrict__ indptr, const int* __restrict__ indices, const float* __restrict__ Q,
+    const float* __restrict__ K, const float* __restrict__ V, long ldq, long ldk, long ldv, long q_head, long k_head,
+    long v_head, float* __restrict__ out, long ldo, long o_head, int F, int Fv, float scale) {
+  constexpr int kU = LPR < 4 ? LPR : 4;  // entries per batch
   const int lane = threadIdx.x & 31, sub = lane / LPR, sl = lane % LPR;
   const unsigned mask = (LPR == 32) ? 0xffffffffu : (((1u << LPR) - 1u) << (sub * LPR));
   const long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
   if (r >= n_rows) return;  // the whole group leaves together
   const long h = blockIdx.y;
-  const float* Qh = Q + h * q_head;
   const float* Kh = K + h * k_head;
   const float* Vh = V + h * v_head;
-  // this lane's features: f .. f + 3 and f2 .. f2 + 3 (each load
-  // instruction of the group reads 16 LPR contiguous bytes of a row)
+  // each load instruction of the group reads 16 LPR contiguous bytes of a row
   const int f = 4 * sl, f2 = f + 4 * LPR;
-  const float* qr = Qh + r * ldq;
-  const float4 q0 = ld4_live(qr, f, F), q1 = ld4_live(qr, f2, F);
-  const int rb = __ldg(indptr + r), re = __ldg(indptr + r + 1);
-  float m = -INFINITY, l = 0.f;
-  float4 acc0 = make_float4(0.f, 0.f, 0.f, 0.f), acc1 = acc0;
-#pragma unroll 1
-  for (int b0 = rb; b0 < re; b0 += 2) {
-    const bool v1 = b0 + 1 < re;
-    const int c0 = __ldg(indices + b0), c1 = v1 ? __ldg(indices + b0 + 1) : c0;
-    const float* k0 = Kh + (long)c0 * ldk;
-    const float* k1 = Kh + (long)c1 * ldk;
-    const float* w0 = Vh + (long)c0 * ldv;
-    const float* w1 = Vh + (long)c1 * ldv;
-    const float4 ka0 = ld4_live(k0, f, F), kb0 = ld4_live(k0, f2, F);
-    const float4 ka1 = ld4_live(k1, f, F), kb1 = ld4_live(k1, f2, F);
-    const float4 va0 = ld4_live(w0, f, Fv), vb0 = ld4_live(w0, f2, Fv);
-    const float4 va1 = ld4_live(w1, f, Fv), vb1 = ld4_live(w1, f2, Fv);
-    const float s0 = dot4(q0, ka0) + dot4(q1, kb0);
-    const float s1 = dot4(q0, ka1) + dot4(q1, kb1);
-    // transposing butterfly: the upper half of the group keeps entry 1
-    const bool up = (sl & (LPR / 2)) != 0;
-    float t = (up ? s1 : s0) + __shfl_xor_sync(mask, up ? s0 : s1, LPR / 2);
+  const Feat8 q = load8<kMask>(Q + h * q_head + r * ldq, f, f2, F);
+  const int rb = __ldg(indptr + r), n = __ldg(indptr + r + 1) - rb;
+  // this lane's entry of a batch: the halving strides' bits of its index
+  int e = 0;
 #pragma unroll
-    for (int o = LPR / 4; o > 0; o >>= 1) t += __shfl_xor_sync(mask, t, o);
-    const float e0 = scale * __shfl_sync(mask, t, 0, LPR);
-    const float e1 = v1 ? scale * __shfl_sync(mask, t, LPR / 2, LPR) : -INFINITY;
-    const float mn = fmaxf(m, fmaxf(e0, e1));
-    const float alpha = expf(m - mn);  // 0 for the first batch (m = -inf)
-    const float p0 = expf(e0 - mn), p1 = expf(e1 - mn);
-    l = l * alpha + p0 + p1;
-    acc0 = make_float4(acc0.x * alpha + p0 * va0.x + p1 * va1.x, acc0.y * alpha + p0 * va0.y + p1 * va1.y,
-                       acc0.z * alpha + p0 * va0.z + p1 * va1.z, acc0.w * alpha + p0 * va0.w + p1 * va1.w);
-    acc1 = make_float4(acc1.x * alpha + p0 * vb0.x + p1 * vb1.x, acc1.y * alpha + p0 * vb0.y + p1 * vb1.y,
-                       acc1.z * alpha + p0 * vb0.z + p1 * vb1.z, acc1.w * alpha + p0 * vb0.w + p1 * vb1.w);
-    m = mn;
+  for (int m = kU, hw = LPR / 2; m > 1; m >>= 1, hw >>= 1)
+    if (sl & hw) e += m / 2;
+  float m = -INFINITY, l = 0.f;
+  f32x2 acc[4] = {0, 0, 0, 0};
+  auto col_at = [&](int i) { return __ldg(indices + rb + min(i, n - 1)); };  // past the row: a valid entry, weight 0
+  int cl = n > 0 ? col_at(sl) : 0;
+#pragma unroll 1
+  for (int c0 = 0; c0 < n; c0 += LPR) {
+    const int cl1 = col_at(c0 + LPR + sl);
+#pragma unroll 1
+    for (int b0 = 0; b0 < min(LPR, n - c0); b0 += kU) {
+      Feat8 k[kU], v[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const long c = __shfl_sync(mask, cl, b0 + u, LPR);
+        k[u] = load8<kMask>(Kh + c * ldk, f, f2, F);
+        // features past Fv are never stored
+        v[u] = load8<(kMask == 0 ? 0 : 1)>(Vh + c * ldv, f, f2, Fv);
+      }
+      float s[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        f32x2 d = mul2(q.v[0], k[u].v[0]);
+#pragma unroll
+        for (int w = 1; w < 4; ++w) d = fma2(q.v[w], k[u].v[w], d);
+        const float2 p = unpack2(d);
+        s[u] = p.x + p.y;
+      }
+      // transposing butterfly: this lane keeps entry e's score
+#pragma unroll
+      for (int w = kU, hw = LPR / 2; w > 1; w >>= 1, hw >>= 1) {
+        const bool up = (sl & hw) != 0;
+#pragma unroll
+        for (int i = 0; i < w / 2; ++i) {
+          const float send = up ? s[i] : s[i + w / 2];
+          const float keep = up ? s[i + w / 2] : s[i];
+          s[i] = keep + __shfl_xor_sync(mask, send, hw);
+        }
+      }
+#pragma unroll
+      for (int o = LPR / (2 * kU); o > 0; o >>= 1) s[0] += __shfl_xor_sync(mask, s[0], o);
+      const float t = c0 + b0 + e < n ? scale * s[0] : -INFINITY;
+      float mn = fmaxf(m, t);
+#pragma unroll
+      for (int w = kU, hw = LPR / 2; w > 1; w >>= 1, hw >>= 1) mn = fmaxf(mn, __shfl_xor_sync(mask, mn, hw));
+      const float ref = mn == -INFINITY ? 0.f : mn;  // only -inf scores so far: weights 0
+      const float alpha = expf(m - ref);             // 0 for the first batch (m = -inf)
+      const float p = expf(t - ref);
+      l = fmaf(l, alpha, p);
+      m = mn;
+      const f32x2 a2 = pack2(alpha, alpha);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) acc[w] = mul2(acc[w], a2);
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        // a lane that holds entry u: its index's halving bits spell u
+        int src = 0;
+#pragma unroll
+        for (int w = kU, hw = LPR / 2, x = u; w > 1; w >>= 1, hw >>= 1) {
+          if (x >= w / 2) {
+            src += hw;
+            x -= w / 2;
+          }
+        }
+        const float pu = __shfl_sync(mask, p, src, LPR);
+        const f32x2 p2 = pack2(pu, pu);
+        // entries past the row add nothing (a weight of 0 would still turn an
+        // infinite V into NaN; predicates on their loads cost a third of the
+        // kernel's rate)
+        if (u == 0 || c0 + b0 + u < n) {
+#pragma unroll
+          for (int w = 0; w < 4; ++w) acc[w] = fma2(p2, v[u].v[w], acc[w]);
+        }
+      }
+    }
+    cl = cl1;
   }
+  // the entry slots' sums
+#pragma unroll
+  for (int w = kU, hw = LPR / 2; w > 1; w >>= 1, hw >>= 1) l += __shfl_xor_sync(mask, l, hw);
   // a row without entries attends to nothing: zeros
-  const float inv = l > 0.f ? 1.f / l : 0.f;
+  const float inv = n > 0 ? 1.f / l : 0.f;
   float* orow = out + h * o_head + r * ldo;
-  st_row4(orow, f, Fv, make_float4(acc0.x * inv, acc0.y * inv, acc0.z * inv, acc0.w * inv));
-  st_row4(orow, f2, Fv, make_float4(acc1.x * inv, acc1.y * inv, acc1.z * inv, acc1.w * inv));
+  float2 o[4];
+#pragma unroll
+  for (int w = 0; w < 4; ++w) o[w] = unpack2(acc[w]);
+  st_row4(orow, f, Fv, make_float4(o[0].x * inv, o[0].y * inv, o[1].x * inv, o[1].y * inv));
+  st_row4(orow, f2, Fv, make_float4(o[2].x * inv, o[2].y * inv, o[3].x * inv, o[3].y * inv));
+}
+
+template <int LPR>
+static cudaError_t launch_att_t(dim3 grid, cudaStream_t st, int n_rows, const int* indptr, const int* indices,
+                                const float* Q, const float* K, const float* V, long ldq, long ldk, long ldv,
+                                long q_head, long k_head, long v_head, float* out, long ldo, long o_head, int F, int Fv,
+                                float scale) {
+#define STILE_ATT(MASK)                                                                                        \
+  sparse_attention_kernel<LPR, MASK><<<grid, kAttThreads, 0, st>>>(n_rows, indptr, indices, Q, K, V, ldq, ldk, ldv, \
+                                                                   q_head, k_head, v_head, out, ldo, o_head, F, Fv, scale)
+  if (F == 8 * LPR && Fv == 8 * LPR) STILE_ATT(0);
+  else if (F % 4 == 0) STILE_ATT(1);
+  else STILE_ATT(2);
+#undef STILE_ATT
+  return cudaGetLastError();
 }
 
 cudaError_t launch_sparse_attention(int n_rows, const int* indptr, const int* indices, const float* Q,
@@ -91,18 +185,16 @@ cudaError_t launch_sparse_attention(int n_rows, const int* indptr, const int* in
   const int width = F > Fv ? F : Fv;  // features per lane: 8; lanes: the power of two covering the wider row
   int lpr = 2;
   while (8 * lpr < width) lpr <<= 1;
-  const dim3 grid((unsigned)(((long)n_rows * lpr + 255) / 256), (unsigned)heads);
-#define STILE_ATT(L)                                                                                              \
-  sparse_attention_kernel<L><<<grid, 256, 0, st>>>(n_rows, indptr, indices, Q, K, V, ldq, ldk, ldv, q_head, k_head, \
-                                                   v_head, out, ldo, o_head, F, Fv, scale)
+  const dim3 grid((unsigned)(((long)n_rows * lpr + kAttThreads - 1) / kAttThreads), (unsigned)heads);
+#define STILE_ATT_ARGS grid, st, n_rows, indptr, indices, Q, K, V, ldq, ldk, ldv, q_head, k_head, v_head, out, ldo, \
+                       o_head, F, Fv, scale
   switch (lpr) {
-    case 2: STILE_ATT(2); break;
-    case 4: STILE_ATT(4); break;
-    case 8: STILE_ATT(8); break;
-    default: STILE_ATT(16); break;
+    case 2: return launch_att_t<2>(STILE_ATT_ARGS);
+    case 4: return launch_att_t<4>(STILE_ATT_ARGS);
+    case 8: return launch_att_t<8>(STILE_ATT_ARGS);
+    default: return launch_att_t<16>(STILE_ATT_ARGS);
   }
-#undef STILE_ATT
-  return cudaGetLastError();
+#undef STILE_ATT_ARGS
 }
 
 }  // namespace stile
