@@ -649,7 +649,11 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) spmm_tc_kernel(SpmmArgs p
 // and few registers leave room for many warps per SM.
 // kFull: N % (4 * VEC * LPR) == 0, every lane's features are in range
 // (otherwise a float4 that starts past N reads as zero).
-// kOff32: every B row offset col * ldb fits in 32 bits.
+// kAddr: how a B row's address is formed: kOff32, every row offset col * ldb
+// fits in 31 bits; kRow32, a row is shorter than 4 GB (one 32 x 32 + 64 bit
+// multiply-add a row: a graph at N = 200 117 us where the 64-bit product took
+// 126; full rows gain another 2 to 10% from the 31-bit offset, which leaves a
+// register free); kRow64, any.
 // kSpanY: blockIdx.y takes features [y span, (y + 1) span) (a wide B over
 // few groups; span = p.ell_fc_span, a multiple of the pass width).
 // kHeads: a batched run (blockIdx.z = head offsets B, C and the values).
@@ -662,7 +666,18 @@ __device__ __forceinline__ int3 ell_record(const int2* __restrict__ ent, const f
   return make_int3(e.x, __float_as_int(__ldcs(val + i)), e.y);
 }
 
-template <int LPR, int VEC, bool kFull, bool kOff32, bool kSpanY = false, bool kHeads = false>
+enum { kOff32, kRow32, kRow64 };
+
+// row `row` of an operand of `ld` elements a row
+template <int kAddr, typename T>
+__device__ __forceinline__ const T* row_at(const T* from, long ld, int row) {
+  if (kAddr == kRow64) return from + (long)row * ld;
+  if (kAddr == kOff32) return from + (unsigned)(row * (int)ld);
+  return reinterpret_cast<const T*>(reinterpret_cast<const char*>(from) +
+                                    (unsigned long long)(unsigned)row * (unsigned)(ld * (long)sizeof(T)));
+}
+
+template <int LPR, int VEC, bool kFull, int kAddr, bool kSpanY = false, bool kHeads = false>
 __global__ void __launch_bounds__(256, 5) spmm_ell_seg_kernel(SpmmArgs p) {
   constexpr int kBatch = 4 / VEC;  // entries per batch: 4 float4 in flight per lane
   // Launched dependent on the previous kernel.  When that is the zero-rows
@@ -686,7 +701,6 @@ __global__ void __launch_bounds__(256, 5) spmm_ell_seg_kernel(SpmmArgs p) {
   const int2* __restrict__ ent = p.ell_entry + p0;
   const float* __restrict__ val = p.ell_val + head * p.ell_n_pos + p0;
   const int N = p.N;
-  const int ldb32 = (int)p.ldb;
   // records are read once: streaming loads leave L2 to the B rows
   auto rec = [&](int i) { return ell_record(ent, val, i, n); };
   for (int fc = kSpanY ? blockIdx.y * p.ell_fc_span : 0;
@@ -710,13 +724,13 @@ __global__ void __launch_bounds__(256, 5) spmm_ell_seg_kernel(SpmmArgs p) {
           const int c = __shfl_sync(mask, mcur.x, b0 - c0 + u, LPR);
           // records past n hold column 0: a valid row, multiplied by 0
           if (kFull) {
-            const float* row = kOff32 ? Bf + (unsigned)(c * ldb32) : Bf + (long)c * p.ldb;
+            const float* row = row_at<kAddr>(Bf, p.ldb, c);
 #pragma unroll
             for (int w = 0; w < VEC; ++w) bv[u][w] = ldg4(row + 4 * LPR * w);
           } else {
             // float4 past N read as zero; padding features inside the last
             // live float4 only reach features that are never stored
-            const float* row = p.B + head * p.b_head_stride + (long)c * p.ldb;
+            const float* row = row_at<kAddr>(p.B + head * p.b_head_stride, p.ldb, c);
 #pragma unroll
             for (int w = 0; w < VEC; ++w) bv[u][w] = ld4_pad(row, f + 4 * LPR * w, N);
           }
@@ -883,7 +897,7 @@ cudaError_t launch_permute_ids(const int* in, long n, const int* perm, int* out,
 // The same entry stream over a bf16 B: each lane covers 8 features with one
 // 16-byte load (half the gathered bytes of fp32 rows), converts them to
 // fp32 and accumulates in fp32; 4 entries' rows in flight per lane.
-template <int LPR, bool kFull, bool kOff32, bool kSpanY = false>
+template <int LPR, bool kFull, int kAddr, bool kSpanY = false>
 __global__ void __launch_bounds__(256, 4) spmm_ell_seg_bf16_kernel(SpmmArgs p) {
   constexpr int kBatch = 4;
   static_assert(LPR % kBatch == 0, "batches stay inside one record block");
@@ -909,7 +923,6 @@ __global__ void __launch_bounds__(256, 4) spmm_ell_seg_bf16_kernel(SpmmArgs p) {
   const uint16_t* __restrict__ B16 = reinterpret_cast<const uint16_t*>(p.B) + blockIdx.z * p.b_head_stride;
   float* __restrict__ Ch = p.C + blockIdx.z * p.c_head_stride;
   const int N = p.N;
-  const int ldb32 = (int)p.ldb;
   // records are read once: streaming loads leave L2 to the B rows
   auto rec = [&](int i) { return ell_record(ent, val, i, n); };
   for (int fc = kSpanY ? blockIdx.y * p.ell_fc_span : 0;
@@ -927,7 +940,7 @@ __global__ void __launch_bounds__(256, 4) spmm_ell_seg_bf16_kernel(SpmmArgs p) {
         for (int u = 0; u < kBatch; ++u) {
           const int c = __shfl_sync(mask, mcur.x, b0 - c0 + u, LPR);
           // records past n hold column 0: a valid row, multiplied by 0
-          const uint16_t* row = kOff32 ? B16 + (unsigned)(c * ldb32) : B16 + (long)c * p.ldb;
+          const uint16_t* row = row_at<kAddr>(B16, p.ldb, c);
           bv[u] = kFull ? ldg_u4(row + f) : ld_row8_bf16(row, f, N);
         }
 #pragma unroll
@@ -1328,16 +1341,34 @@ static dim3 ell_grid(SpmmArgs& p, int groups_per_block, int pass) {
   return dim3((unsigned)gx, (unsigned)gy, (unsigned)std::max(1, p.heads));
 }
 
+// every row offset of B in 31 bits; a row's bytes in 32
+static bool b_off32(const SpmmArgs& p) { return (long)p.K * p.ldb < (1L << 31); }
+static bool b_row32(const SpmmArgs& p) { return p.ldb * (p.b_bf16 ? 2 : 4) < (1L << 32); }
+
+template <int LPR, int VEC, bool kFull, int kAddr>
+static cudaError_t launch_ell_addr(const SpmmArgs& p, dim3 grid, cudaStream_t st) {
+  if (grid.z > 1)
+    return launch_dependent(spmm_ell_seg_kernel<LPR, VEC, kFull, kAddr, true, true>, grid, dim3(256), 0, st, p);
+  if (grid.y > 1)
+    return launch_dependent(spmm_ell_seg_kernel<LPR, VEC, kFull, kAddr, true>, grid, dim3(256), 0, st, p);
+  return launch_dependent(spmm_ell_seg_kernel<LPR, VEC, kFull, kAddr>, grid, dim3(256), 0, st, p);
+}
+
+// (the 64-bit row stride: one general variant per group width)
+template <int LPR, int VEC, bool kFull>
+static cudaError_t launch_ell_seg(const SpmmArgs& p, dim3 grid, cudaStream_t st) {
+  if (!b_row32(p))
+    return launch_dependent(spmm_ell_seg_kernel<LPR, VEC, false, kRow64, true, true>, grid, dim3(256), 0, st, p);
+  if (kFull && b_off32(p)) return launch_ell_addr<LPR, VEC, kFull, kFull ? kOff32 : kRow32>(p, grid, st);
+  return launch_ell_addr<LPR, VEC, kFull, kRow32>(p, grid, st);
+}
+
 template <int LPR>
 struct EllLaunch {
   static cudaError_t run(SpmmArgs p, cudaStream_t st) {
     if (p.ell_n_groups == 0) return cudaSuccess;
     const dim3 grid = ell_grid(p, 256 / LPR, 4 * LPR);
-    if (grid.z > 1)
-      return launch_dependent(spmm_ell_seg_kernel<LPR, 1, false, false, true, true>, grid, dim3(256), 0, st, p);
-    if (grid.y > 1)
-      return launch_dependent(spmm_ell_seg_kernel<LPR, 1, false, false, true>, grid, dim3(256), 0, st, p);
-    return launch_dependent(spmm_ell_seg_kernel<LPR, 1, false, false>, grid, dim3(256), 0, st, p);
+    return launch_ell_seg<LPR, 1, false>(p, grid, st);
   }
 };
 
@@ -1348,27 +1379,25 @@ template <int LPR>
 struct EllNarrowLaunch {
   static cudaError_t run(SpmmArgs p, cudaStream_t st) {
     const dim3 grid = ell_grid(p, 256 / LPR, 8 * LPR);
-    const bool full = p.N % (8 * LPR) == 0;
-    if (grid.z > 1)
-      return full ? launch_dependent(spmm_ell_seg_kernel<LPR, 2, true, false, true, true>, grid, dim3(256), 0, st, p)
-                  : launch_dependent(spmm_ell_seg_kernel<LPR, 2, false, false, true, true>, grid, dim3(256), 0, st, p);
-    if (grid.y > 1)
-      return full ? launch_dependent(spmm_ell_seg_kernel<LPR, 2, true, false, true>, grid, dim3(256), 0, st, p)
-                  : launch_dependent(spmm_ell_seg_kernel<LPR, 2, false, false, true>, grid, dim3(256), 0, st, p);
     // (4 entries per batch at 4 blocks per SM measured slower at N = 41,
     // 159 against 154 us on the GCN graph)
-    return full ? launch_dependent(spmm_ell_seg_kernel<LPR, 2, true, false>, grid, dim3(256), 0, st, p)
-                : launch_dependent(spmm_ell_seg_kernel<LPR, 2, false, false>, grid, dim3(256), 0, st, p);
+    return p.N % (8 * LPR) == 0 ? launch_ell_seg<LPR, 2, true>(p, grid, st) : launch_ell_seg<LPR, 2, false>(p, grid, st);
   }
 };
+
+template <int LPR, bool kFull>
+static cudaError_t launch_ell_seg_bf16(const SpmmArgs& p, dim3 grid, cudaStream_t st) {
+  if (!b_row32(p))
+    return launch_dependent(spmm_ell_seg_bf16_kernel<LPR, false, kRow64, true>, grid, dim3(256), 0, st, p);
+  if (grid.y > 1) return launch_dependent(spmm_ell_seg_bf16_kernel<LPR, kFull, kRow32, true>, grid, dim3(256), 0, st, p);
+  return launch_dependent(spmm_ell_seg_bf16_kernel<LPR, kFull, kRow32>, grid, dim3(256), 0, st, p);
+}
 
 template <int LPR>
 struct EllBf16Launch {
   static cudaError_t run(SpmmArgs p, cudaStream_t st) {
     const dim3 grid = ell_grid(p, 256 / LPR, 8 * LPR);
-    if (grid.y > 1)
-      return launch_dependent(spmm_ell_seg_bf16_kernel<LPR, false, false, true>, grid, dim3(256), 0, st, p);
-    return launch_dependent(spmm_ell_seg_bf16_kernel<LPR, false, false>, grid, dim3(256), 0, st, p);
+    return launch_ell_seg_bf16<LPR, false>(p, grid, st);
   }
 };
 
@@ -1383,28 +1412,13 @@ static int lpr_for_bf16(int N) {
 cudaError_t launch_ell(const SpmmArgs& args, cudaStream_t st) {
   if (args.ell_n_groups == 0) return cudaSuccess;
   SpmmArgs p = args;
-  const bool off32 = (long)p.K * p.ldb < (1L << 31);
   if (p.b_bf16) {
-    if (p.N % 128 == 0) {
-      // 16-lane sub-groups of 8 features per lane (two groups per warp)
-      const dim3 grid = ell_grid(p, 16, 128);
-      if (grid.y > 1)
-      return launch_dependent(spmm_ell_seg_bf16_kernel<16, true, false, true>, grid, dim3(256), 0, st, p);
-      else if (off32) return launch_dependent(spmm_ell_seg_bf16_kernel<16, true, true>, grid, dim3(256), 0, st, p);
-      return launch_dependent(spmm_ell_seg_bf16_kernel<16, true, false>, grid, dim3(256), 0, st, p);
-    }
+    // 16-lane sub-groups of 8 features per lane (two groups per warp)
+    if (p.N % 128 == 0) return launch_ell_seg_bf16<16, true>(p, ell_grid(p, 16, 128), st);
     return dispatch_lpr<EllBf16Launch>(lpr_for_bf16(p.N), p, st);
   }
-  if (p.N % 128 == 0) {
-    // 16-lane sub-groups of 8 features per lane (two groups per warp)
-    const dim3 grid = ell_grid(p, 16, 128);
-    if (grid.z > 1)
-      return launch_dependent(spmm_ell_seg_kernel<16, 2, true, false, true, true>, grid, dim3(256), 0, st, p);
-    if (grid.y > 1)
-      return launch_dependent(spmm_ell_seg_kernel<16, 2, true, false, true>, grid, dim3(256), 0, st, p);
-    else if (off32) return launch_dependent(spmm_ell_seg_kernel<16, 2, true, true>, grid, dim3(256), 0, st, p);
-    return launch_dependent(spmm_ell_seg_kernel<16, 2, true, false>, grid, dim3(256), 0, st, p);
-  }
+  // 16-lane sub-groups of 8 features per lane (two groups per warp)
+  if (p.N % 128 == 0) return launch_ell_seg<16, 2, true>(p, ell_grid(p, 16, 128), st);
   if (p.N < 128) {
     int lpr = 4;
     while (lpr < (p.N + 7) / 8) lpr <<= 1;

@@ -7,6 +7,7 @@ import torch
 import oracle.semantics as S
 from stile_gb300 import device as D
 from stile_gb300 import synthetic as syn
+from stile_gb300.api import PlanConfig, SpmmOperator
 from stile_gb300.ops import DeviceSddmmPlan, dense_operand, dense_operand_bf16
 from stile_gb300.planner import search_sddmm
 
@@ -52,3 +53,18 @@ def test_scores_of_disjoint_and_overlapping_tiles(shared, F, bf16):
     if shared and not bf16:     # the 1D kernel's fp32 sums, not the block kernel's split products
         e = dev.blk_out[:5]
         assert np.allclose(out.cpu().numpy()[e], ref[e], rtol=1e-6, atol=F * 1e-7)
+
+
+@pytest.mark.parametrize("N,dtype", [(128, torch.float32), (41, torch.float32), (200, torch.float32),
+                                     (256, torch.bfloat16), (72, torch.bfloat16)])
+def test_product_of_rows_far_apart(N, dtype):
+    """A view whose row stride makes every row offset exceed 31 bits of
+    elements gives what the packed rows give (the same sums in the same
+    order, but for atomic adds)."""
+    A = syn.community_graph(n=640, target_nnz=9000, seed=4, max_deg=200)
+    op = SpmmOperator(A, N, PlanConfig())
+    B = torch.randn(A.shape[1], N, device="cuda").to(dtype)
+    ld = (1 << 31) // 600 // 8 * 8          # 640 rows of 3.58M elements: 2.29e9 elements
+    far = torch.empty(A.shape[1] * ld, dtype=dtype, device="cuda").as_strided((A.shape[1], N), (ld, 1))
+    far.copy_(B)
+    assert torch.allclose(op(far), op(B), rtol=1e-5, atol=1e-5)
