@@ -136,6 +136,19 @@ static inline cudaError_t launch_dependent(void (*k)(KArgs...), dim3 grid, dim3 
   return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// How a gathered row's address is formed: kOff32, every row offset row * ld fits
+// in 31 bits; kRow32, a row is shorter than 4 GB; kRow64, any.
+enum { kOff32, kRow32, kRow64 };
+
+// row `row` of an operand of `ld` elements a row
+template <int kAddr, typename T>
+__device__ __forceinline__ const T* row_at(const T* from, long ld, int row) {
+  if (kAddr == kRow64) return from + (long)row * ld;
+  if (kAddr == kOff32) return from + (unsigned)(row * (int)ld);
+  return reinterpret_cast<const T*>(reinterpret_cast<const char*>(from) +
+                                    (unsigned long long)(unsigned)row * (unsigned)(ld * (long)sizeof(T)));
+}
+
 // bf16 rows: 16-byte vectors of 8 features
 __device__ __forceinline__ uint4 ldg_u4(const void* p) {
   return __ldg(reinterpret_cast<const uint4*>(p));

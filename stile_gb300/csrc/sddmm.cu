@@ -256,7 +256,7 @@ constexpr int kRunBlocks = 6;  // resident 256-thread blocks per SM (register bu
 
 // kOne: F <= 4 VEC LPR (one pass; the X row stays in registers).
 // kFull: F == 4 VEC LPR exactly (no masking at all).
-template <int LPR, int VEC, int U, int MINB, bool kYb, bool kOne, bool kFull, bool kXb = false>
+template <int LPR, int VEC, int U, int MINB, bool kYb, bool kOne, bool kFull, bool kXb, int kAddr>
 __global__ void __launch_bounds__(256, MINB) sddmm_run_kernel(int n_groups, const int* __restrict__ gptr,
                                                                 const int* __restrict__ grow,
                                                                 const int* __restrict__ cols,
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(256, MINB) sddmm_run_kernel(int n_groups, cons
     }
   };
   auto load_y = [&](int c, int f, float4 (&y)[VEC]) {
-    const TY* row = Y + (long)c * ldy;
+    const TY* row = row_at<kAddr>(Y, ldy, c);
     if constexpr (kYb) {
       bf16x8_to_f32(kFull ? ldg_u4(row + f) : ld_row8_bf16(row, f, F), y[0], y[1]);
     } else {
@@ -366,16 +366,20 @@ static cudaError_t launch_runs_t(int grid, bool one, bool full, cudaStream_t st,
   // flight per group at 5 blocks per SM: a narrow row is few bytes, and the
   // gathers are bound by the bytes in flight
   constexpr int U = L <= 8 ? 4 : kRunU, MINB = L <= 8 ? 5 : kRunBlocks;
-  if (full)
-    return launch_dependent(sddmm_run_kernel<L, 2, U, MINB, kYb, true, true, kXb>, dim3((unsigned)grid), dim3(256), 0,
-                            st, n_groups, gptr, grow, cols, outs, X, ldx, Y, ldy, out, F);
-  if (one)
-    return launch_dependent(sddmm_run_kernel<L, 2, U, MINB, kYb, true, false, kXb>, dim3((unsigned)grid), dim3(256),
-                            0, st, n_groups, gptr, grow, cols, outs, X, ldx, Y, ldy, out, F);
-  // several passes: 4 rows and the X slice in flight per pass (2 rows at 6
-  // blocks: 264 against 206 us at F = 4096 on a 768 x 3072 weight)
-  return launch_dependent(sddmm_run_kernel<L, 2, 4, 4, kYb, false, false, kXb>, dim3((unsigned)grid), dim3(256), 0, st,
-                          n_groups, gptr, grow, cols, outs, X, ldx, Y, ldy, out, F);
+#define STILE_RUN_KERNEL(u, b, o, f, a)                                                                       \
+  launch_dependent(sddmm_run_kernel<L, 2, u, b, kYb, o, f, kXb, a>, dim3((unsigned)grid), dim3(256), 0, st, n_groups, \
+                   gptr, grow, cols, outs, X, ldx, Y, ldy, out, F)
+  // one pass: the row's address is a 32 x 32 + 64 bit multiply-add (rows
+  // shorter than 4 GB; bf16 rows of 64 features 53 -> 47 us on a 2M-entry mask)
+  const bool row32 = ldy * (kYb ? 2 : 4) < (1L << 32);
+  if (full && row32) return STILE_RUN_KERNEL(U, MINB, true, true, kRow32);
+  if (one && row32) return STILE_RUN_KERNEL(U, MINB, true, false, kRow32);
+  // several passes (or longer rows): 4 rows and the X slice in flight per pass
+  // (2 rows at 6 blocks: 264 against 206 us at F = 4096 on a 768 x 3072
+  // weight); the addresses are formed once per entry and pass, and the 64-bit
+  // product was the faster one (206 against 215 us)
+  return STILE_RUN_KERNEL(4, 4, false, false, kRow64);
+#undef STILE_RUN_KERNEL
 }
 
 cudaError_t launch_sddmm_runs(int n_groups, const int* gptr, const int* grow, const int* cols, const int* outs,

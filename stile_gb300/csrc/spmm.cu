@@ -666,17 +666,6 @@ __device__ __forceinline__ int3 ell_record(const int2* __restrict__ ent, const f
   return make_int3(e.x, __float_as_int(__ldcs(val + i)), e.y);
 }
 
-enum { kOff32, kRow32, kRow64 };
-
-// row `row` of an operand of `ld` elements a row
-template <int kAddr, typename T>
-__device__ __forceinline__ const T* row_at(const T* from, long ld, int row) {
-  if (kAddr == kRow64) return from + (long)row * ld;
-  if (kAddr == kOff32) return from + (unsigned)(row * (int)ld);
-  return reinterpret_cast<const T*>(reinterpret_cast<const char*>(from) +
-                                    (unsigned long long)(unsigned)row * (unsigned)(ld * (long)sizeof(T)));
-}
-
 template <int LPR, int VEC, bool kFull, int kAddr, bool kSpanY = false, bool kHeads = false>
 __global__ void __launch_bounds__(256, 5) spmm_ell_seg_kernel(SpmmArgs p) {
   constexpr int kBatch = 4 / VEC;  // entries per batch: 4 float4 in flight per lane
