@@ -169,10 +169,10 @@ __device__ __forceinline__ uint32_t a_img_off(int m, int k) {
 // least loaded CTA) and stores every CTA's k-steps contiguously, so a CTA's
 // work is the step range [s_beg, s_beg + S), walked once per 128-feature
 // slice; its units are (slice, accumulation unit) pairs in that order.
-//  * Seven gathering warps.  A stage is kSpw consecutive k-steps: 1 at 128
+//  * Four gathering warps.  A stage is kSpw consecutive k-steps: 1 at 128
 //    fp32 features a row, 2 or 4 where 64 or 32 features (or 16-bit rows)
 //    leave a warp-wide 16-byte load room for 2 or 4 rows, so every stage is 16
-//    loads of 512 bytes.  Warp w takes the stages w, w + 7, ...  It holds a
+//    loads of 512 bytes.  Warp w takes the stages w, w + 4, ...  It holds a
 //    stage's rows in registers, converts them into its operand slot (A: the
 //    features are M = 128) and at once loads its next stage's rows, which are
 //    in flight while the MMA warp and the epilogue work.  The rows never pass
@@ -181,28 +181,30 @@ __device__ __forceinline__ uint32_t a_img_off(int m, int k) {
 //    of that, where the cp.async stage of an earlier build added a write and a
 //    read of the whole fp32 row.  Column ids and value images come by cp.async
 //    two and one stages ahead.
-//    14 gathering warps at 128 registers per SM measured faster than 16 at 96
-//    (spilled) and than 16 warps that each owned accumulators, whose sums also
-//    depended on the split.
+//    16 gathering warps per SM at 96 registers spilled; 16 warps that each
+//    owned accumulators made the sums depend on the split.
 //  * The MMA warp takes the stages in order and accumulates the
 //    k-steps of a unit one after another into one of kAccBufs 16-column
 //    accumulators, so the sums do not depend on the warps' timing.
 //  * Epilogue, by the gathering warps: before its stage in unit y a warp
-//    writes its share (a quarter of the features, half of the tile's rows;
-//    warp 3 both halves) of every unit up to y - kLag - 1, whose MMAs are long
-//    done.
-// Bound by the stages' own chain (wait, convert, issue, fence: about 1,400
-// cycles without contention, 14 of them in turn on an SM), not by L2 or the
-// tensor pipe.  Forward of a graph (row tiles included), before -> after:
-// 169,343 nodes, 1.17M nonzeros: N = 128 64 -> 57 us, N = 41 80 -> 64 us,
-// N = 256 in bf16 121 -> 101 us; 50,000 nodes, 2.4M nonzeros: N = 128 73 -> 62
-// us, N = 41 70 -> 54 us; a 4096^2 matrix in split-bf16 22 -> 12 us; a pruned
-// 3072 x 768 weight at N = 4096 in bf16 223 -> 136 us.
+//    writes its quarter of the features of every unit up to y - kLag - 1,
+//    whose MMAs are long done.
+// Bound by two chains, not by L2 or the tensor pipe: a stage's (wait, convert,
+// issue, fence: about 1,400 cycles without contention) and the MMA warp's
+// (about 350 cycles a stage, most of it barrier latency).  Three CTAs of 4 + 1
+// warps per SM give the second chain three times; two of 7 + 1 warps left the
+// gathering warps waiting 60% of their time for slots over wide B (pruned
+// weight, N = 4096 in bf16: 133 against 119 us).  Forward of a graph (row tiles
+// included), before -> after: 169,343 nodes, 1.17M nonzeros: N = 128 64 -> 58
+// us, N = 41 80 -> 61 us, N = 256 in bf16 121 -> 97 us; 50,000 nodes, 2.4M
+// nonzeros: N = 128 73 -> 63 us, N = 41 70 -> 50 us; a 4096^2 matrix in
+// split-bf16 22 -> 13 us; a pruned 3072 x 768 weight at N = 4096 in bf16
+// 223 -> 119 us, 768 x 3072 in fp32 156 -> 109 us.
 // Every wait is bounded; a wait that gives up sets the error flag and ends
 // that warp's work, and the others then end at their next (bounded) wait.
-constexpr int kTcWarps = 7;                        // gathering warps
+constexpr int kTcWarps = 4;                        // gathering warps
 constexpr int kTcThreads = (kTcWarps + 1) * kWarp; // and the MMA warp
-constexpr int kTcCtas = 2;                         // resident CTAs per SM (128 registers a thread)
+constexpr int kTcCtas = 3;                         // resident CTAs per SM (128 registers a thread)
 constexpr int kAccBufs = 8;                        // accumulators of 16 TMEM columns
 // units between a warp's stage and the ones it writes; a warp whose next stage
 // is in unit y has written every unit below y - kLag, so the MMA of unit y or
@@ -265,7 +267,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) spmm_tc_kernel(SpmmArgs p
   const uint32_t drain = acce0 + 8 * kAccBufs, tmem_slot = drain + 8;
 
   // this CTA's first unit, units, first k-step and k-steps
-  const int4 cta = __ldg(p.tc_cta_info + blockIdx.x);
+  const int4 cta = __ldg(p.tc_cta_info + blockIdx.y);
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2 * kTcWarps * kNs; ++s) mbar_init(full0 + 8 * s, 1);
     for (int b = 0; b < kAccBufs; ++b) {
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) spmm_tc_kernel(SpmmArgs p
   const int ub = cta.x, nu = cta.y, s_beg = cta.z, S = cta.w;
   // feature slices of this CTA: blockIdx.y takes [sl0, sl0 + nf) (a wide B
   // spreads its slices over more CTAs than the schedule has)
-  const int sl0 = blockIdx.y * p.tc_slice_per;
+  const int sl0 = blockIdx.x * p.tc_slice_per;
   const int nf = nu > 0 ? min(p.tc_slice_per, p.n_fchunks - sl0) : 0;
   const int Q = (S + kSpw - 1) / kSpw;  // stages per slice
   const int n_units = nu * nf;
@@ -434,7 +436,6 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) spmm_tc_kernel(SpmmArgs p
     // ---- epilogue: the next unit to write, its slice, its meta and output
     // rows (those of the one after it are loaded while it is written)
     const int quarter = warp & 3;
-    const bool half0 = warp < 4, half1 = warp >= 3;  // rows 0-7, 8-15 of the tile
     const int* my_rows = p.tc_unit_rows + (long)ub * 16 + (lane & 15);
     int e = 0, eu = 0, esl = 0;
     int meta = n_units > 0 ? __ldg(p.tc_unit_meta + ub) : 0, rows = n_units > 0 ? __ldg(my_rows) : -1;
@@ -464,8 +465,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtas) spmm_tc_kernel(SpmmArgs p
         const char* Cf = reinterpret_cast<const char*>(p.C + blockIdx.z * p.c_head_stride + f);
         const bool in = (kFull && kRowF == 128) || f < N;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (!live || !(h ? half1 : half0)) continue;
+        for (int h = 0; h < 2; ++h) {  // rows 0-7, 8-15 of the tile
+          if (!live) continue;
           uint32_t r[8];
           tmem_ld8(tmem + (uint32_t)(16 * b + 8 * h) + ((uint32_t)(32 * quarter) << 16), r);
           tmem_wait_ld();
@@ -1210,6 +1211,8 @@ static cudaError_t resident_ctas(K kernel, int threads, size_t smem, int* sms, i
 
 template <int MODE, bool kFull, bool kIn16 = false, int kRowF = 128, bool kBig = false>
 static cudaError_t launch_tc_t(const SpmmArgs& p, cudaStream_t st) {
+  // (the slice groups of a CTA's chunks are neighbours in the launch: the CTAs
+  // with the longest chunks, the schedule's first ones, all start first)
   auto k = spmm_tc_kernel<MODE, kFull, kIn16, kRowF, kBig>;
   constexpr uint32_t kBytes = TcCfg<MODE, kIn16, kRowF>::kBytes;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBytes);
@@ -1220,7 +1223,7 @@ static cudaError_t launch_tc_t(const SpmmArgs& p, cudaStream_t st) {
   e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveout > 100 ? 100 : kCarveout);
   if (e != cudaSuccess) return e;
   if (p.tc_n_chunks == 0 || p.tc_grid == 0) return cudaSuccess;
-  return launch_dependent(k, dim3(p.tc_grid, (p.n_fchunks + p.tc_slice_per - 1) / p.tc_slice_per, std::max(1, p.heads)),
+  return launch_dependent(k, dim3((p.n_fchunks + p.tc_slice_per - 1) / p.tc_slice_per, p.tc_grid, std::max(1, p.heads)),
                           dim3(kTcThreads), kBytes, st, p);
 }
 
@@ -1272,7 +1275,7 @@ int tc_persistent_ctas(int mode) {
 // balances k-steps over tc_grid CTAs; with nf slices a CTA's work is its
 // k-steps times nf.  When that makes the longest CTA much longer than the
 // average over all resident CTAs (a wide B over few chunks), the slices are
-// split over grid.y so that no CTA holds more than about the average.
+// split over grid.x so that no CTA holds more than about the average.
 static int tc_slices_per_cta(const SpmmArgs& p) {
   const int nf = p.n_fchunks;
   if (nf <= 1 || p.tc_max_cta_steps <= 0) return nf;
