@@ -369,11 +369,13 @@ static cudaError_t launch_runs_t(int grid, bool one, bool full, cudaStream_t st,
 #define STILE_RUN_KERNEL(u, b, o, f, a)                                                                       \
   launch_dependent(sddmm_run_kernel<L, 2, u, b, kYb, o, f, kXb, a>, dim3((unsigned)grid), dim3(256), 0, st, n_groups, \
                    gptr, grow, cols, outs, X, ldx, Y, ldy, out, F)
-  // one pass: the row's address is a 32 x 32 + 64 bit multiply-add (rows
-  // shorter than 4 GB; bf16 rows of 64 features 53 -> 47 us on a 2M-entry mask)
-  const bool row32 = ldy * (kYb ? 2 : 4) < (1L << 32);
-  if (full && row32) return STILE_RUN_KERNEL(U, MINB, true, true, kRow32);
-  if (one && row32) return STILE_RUN_KERNEL(U, MINB, true, false, kRow32);
+  // one pass over bf16 rows: the row's address is a 32 x 32 + 64 bit
+  // multiply-add (rows shorter than 4 GB; 64 features on a 2M-entry mask 53 ->
+  // 47 us; fp32 rows, twice the bytes a row, 60 -> 61 us: the 64-bit product)
+  constexpr int kAddr = kYb ? kRow32 : kRow64;
+  const bool fits = !kYb || ldy * 2 < (1L << 32);
+  if (full && fits) return STILE_RUN_KERNEL(U, MINB, true, true, kAddr);
+  if (one && fits) return STILE_RUN_KERNEL(U, MINB, true, false, kAddr);
   // several passes (or longer rows): 4 rows and the X slice in flight per pass
   // (2 rows at 6 blocks: 264 against 206 us at F = 4096 on a 768 x 3072
   // weight); the addresses are formed once per entry and pass, and the 64-bit
