@@ -328,10 +328,12 @@ int stile_spmm_plan_set_dvals_mode(StileSpmmPlan* plan, int32_t mode);
  * Used when A's values change between calls (training the values). */
 int stile_spmm_plan_set_values(StileSpmmPlan* plan, const float* vals, void* stream);
 
-/* The same for the plan of A^T from A's values: vals[nnz] in the forward's
- * numbering (after stile_spmm_plan_set_transpose_ids; no permuted copy of
- * the values is made). */
-int stile_spmm_plan_set_values_forward(StileSpmmPlan* planT, const float* vals, void* stream);
+/* The same for the plan and, in the same launch, for the plan of A^T (after
+ * stile_spmm_plan_set_transpose_ids: from the forward's values, no permuted
+ * copy of them is made), and vals into copy[nnz] (NULL: no copy).  The
+ * plans' tensor tiles must have one mode (else STILE_E_UNSUPPORTED). */
+int stile_spmm_plan_set_values_pair(StileSpmmPlan* plan, StileSpmmPlan* planT, const float* vals, float* copy,
+                                    void* stream);
 
 /* Device-side error flag of a plan's kernels (bounded waits that gave up):
  * synchronises the stream, returns the flag (0 = none) and clears it. */

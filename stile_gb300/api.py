@@ -306,20 +306,17 @@ class SpmmOperator:
         if self._dense is not None:
             W, rows, cols = self._dense
             W[rows, cols] = vals.to(torch.bfloat16)
+        if self._transposed is not None:
+            opT, perm_t = self._transposed
+            if opT._plain is None and opT._dense is None and opT._transposed is None:
+                # nothing but the transposed plan holds its values
+                self._vals_src = self.handle.set_values_pair(opT.handle, vals)
+                opT._vals_src = (self._vals_src, perm_t)
+                return
         self.handle.set_values(vals)
         self._vals_src = vals.clone()
         if self._transposed is not None:
-            opT, perm_t = self._transposed
-            opT._set_values_forward(self._vals, perm_t)
-
-    def _set_values_forward(self, vals, perm):
-        """set_values(vals[perm]) of a transposed operator, without the
-        permuted copy unless something other than the plan needs it."""
-        if self._plain is not None or self._dense is not None or self._transposed is not None:
-            self.set_values(vals[perm])
-            return
-        self.handle.set_values_forward(vals)
-        self._vals_src = (vals, perm)
+            opT.set_values(self._vals_src[perm_t])
 
     @property
     def transposed(self):

@@ -760,9 +760,10 @@ int stile_spmm_values_pack(const StileSpmmPlan* plan, const float* vals, int32_t
   if ((plan->args.tc_n_items && !plan->args.tc_nnz_id) || (plan->args.ell_n_groups && !plan->args.ell_nnz_id))
     return fail(STILE_E_INVALID, "plan was uploaded without nonzero ids");
   uint8_t* pk = static_cast<uint8_t*>(packed);
-  cudaError_t e = stile::launch_pack_values(plan->args, vals, plan->nnz, heads, reinterpret_cast<float*>(pk),
-                                            pk + values_tc_offset(plan, heads), plan->ell_n_slots,
-                                            (long)values_tc_bytes(plan), false, static_cast<cudaStream_t>(stream));
+  const stile::PackPlan to = stile::pack_of(plan->args, plan->ell_n_slots, reinterpret_cast<float*>(pk),
+                                            pk + values_tc_offset(plan, heads), false);
+  cudaError_t e = stile::launch_pack_values(plan->args.tc_mode, to, stile::PackPlan{}, vals, plan->nnz, heads,
+                                            (long)values_tc_bytes(plan), nullptr, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "value pack launch");
   g_launches++;
   return STILE_OK;
@@ -956,30 +957,50 @@ int stile_spmm_backward(const StileSpmmPlan* planT, const float* dC, int64_t ldd
   return STILE_OK;
 }
 
-static int set_values(StileSpmmPlan* plan, const float* vals, bool forward_ids, void* stream) {
-  stile::begin_call();
-  if (!plan || !vals) return fail(STILE_E_INVALID, "null argument");
+static int check_refresh(const StileSpmmPlan* plan, bool forward_ids) {
   if (plan->args.tc_n_chunks && plan->args.tc_mode == STILE_TC_FP8)
     return fail(STILE_E_UNSUPPORTED, "fp8 tensor tiles: new values need a new upload (their row scales change)");
   if ((plan->args.tc_n_items && !plan->args.tc_nnz_id) ||
       (plan->args.ell_n_groups && !plan->args.ell_nnz_id))
     return fail(STILE_E_INVALID, "plan was uploaded without nonzero ids");
   if (forward_ids && !plan->ids_set) return fail(STILE_E_INVALID, "call stile_spmm_plan_set_transpose_ids first");
-  cudaError_t e = stile::launch_pack_values(plan->args, vals, plan->nnz, 1, const_cast<float*>(plan->args.ell_val),
-                                            const_cast<void*>(plan->args.tc_vals), plan->ell_n_slots, 0, forward_ids,
-                                            static_cast<cudaStream_t>(stream));
+  return STILE_OK;
+}
+
+static stile::PackPlan own_values(StileSpmmPlan* plan, bool forward_ids) {
+  return stile::pack_of(plan->args, plan->ell_n_slots, const_cast<float*>(plan->args.ell_val),
+                        const_cast<void*>(plan->args.tc_vals), forward_ids);
+}
+
+int stile_spmm_plan_set_values(StileSpmmPlan* plan, const float* vals, void* stream) {
+  stile::begin_call();
+  if (!plan || !vals) return fail(STILE_E_INVALID, "null argument");
+  if (int rc = check_refresh(plan, false)) return rc;
+  cudaError_t e = stile::launch_pack_values(plan->args.tc_mode, own_values(plan, false), stile::PackPlan{}, vals,
+                                            plan->nnz, 1, 0, nullptr, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "value re-pack launch");
   g_launches++;
   return STILE_OK;
 }
 
-int stile_spmm_plan_set_values(StileSpmmPlan* plan, const float* vals, void* stream) {
-  return set_values(plan, vals, false, stream);
+int stile_spmm_plan_set_values_pair(StileSpmmPlan* plan, StileSpmmPlan* planT, const float* vals, float* copy,
+                                    void* stream) {
+  stile::begin_call();
+  if (!plan || !planT || !vals) return fail(STILE_E_INVALID, "null argument");
+  if (planT->nnz != plan->nnz) return fail(STILE_E_INVALID, "the plans must have the same nonzeros");
+  // a plan without tensor tiles takes either mode
+  if (plan->args.tc_n_ksteps && planT->args.tc_n_ksteps && plan->args.tc_mode != planT->args.tc_mode)
+    return fail(STILE_E_UNSUPPORTED, "the plans must have the same tensor-tile mode");
+  if (int rc = check_refresh(plan, false)) return rc;
+  if (int rc = check_refresh(planT, true)) return rc;
+  const int mode = plan->args.tc_n_ksteps ? plan->args.tc_mode : planT->args.tc_mode;
+  cudaError_t e = stile::launch_pack_values(mode, own_values(plan, false), own_values(planT, true), vals, plan->nnz, 1,
+                                            0, copy, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return cuda_fail(e, "value re-pack launch");
+  g_launches++;
+  return STILE_OK;
 }
 
-int stile_spmm_plan_set_values_forward(StileSpmmPlan* planT, const float* vals, void* stream) {
-  return set_values(planT, vals, true, stream);
-}
 
 int stile_spmm_plan_error_flag(StileSpmmPlan* plan, void* stream, int32_t* flag) {
   if (!plan || !flag) return fail(STILE_E_INVALID, "null argument");

@@ -982,68 +982,90 @@ __global__ void __launch_bounds__(256, 4) spmm_ell_seg_bf16_kernel(SpmmArgs p) {
 // ===========================================================================
 // Bound by memory: it reads every value once (a 32-byte sector per value,
 // their order is the tiles', not the CSR's) and writes every tile value.  A
-// warp takes one k-step of a tensor tile: lane l owns the 8 image elements
-// 8l .. 8l + 7, a byte of the k-step's mask says which of them hold a
-// nonzero, their ids lie one after another, and the lane writes its 16 bytes
-// of the image at once (the other elements are zero).  The ids of the dead
-// elements are never read: a k-step of the 233k-node graph holds 41 nonzeros
-// of 256, 196 bytes of mask and ids in place of 1 KB.  The row-tile values
-// are an array of their own, 4 entries a thread.
+// warp takes kPackSteps k-steps of a tensor tile at a time: lane l owns the 8
+// image elements 8l .. 8l + 7 of each, a byte of the k-step's mask says which
+// of them hold a nonzero, their ids lie one after another, and the lane writes
+// its 16 bytes of the image at once (the other elements are zero).  The ids of
+// the dead elements are never read: a k-step of the 233k-node graph holds 41
+// nonzeros of 256, 196 bytes of mask and ids in place of 1 KB.  The row-tile
+// values are an array of their own, 4 entries a thread.  One launch takes the
+// plan, the plan of the transposed operator (ids in the forward's numbering)
+// and the operator's own copy of the values: blocks [0, a.blocks) the first,
+// [a.blocks, a.blocks + b.blocks) the second, the rest copy.
+// (233k-node graph, 11.4M nonzeros, both plans and the copy: 119 us; a launch
+// each, one k-step a warp and a copy by torch 136 us.)
 constexpr int kPackThreads = 256;
+constexpr int kPackSteps = 2;
+
+// one plan's part: k-steps by the first tc_blocks blocks, row-tile values by
+// the others
 template <int MODE>
-__global__ void __launch_bounds__(kPackThreads) pack_values_kernel(SpmmArgs p, const float* __restrict__ vals, long nnz,
-                                                                   const int* __restrict__ tc_ids,
-                                                                   const int* __restrict__ ell_ids,
-                                                                   float* __restrict__ ell_out,
-                                                                   uint8_t* __restrict__ tc_out, long n_ell,
-                                                                   long tc_head_bytes, int tc_blocks) {
-  const long h = blockIdx.y;
-  const float* __restrict__ hv = vals + h * nnz;
-  if ((int)blockIdx.x < tc_blocks) {
-    const int ks = blockIdx.x * (kPackThreads / kWarp) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (ks >= p.tc_n_ksteps) return;
-    const unsigned m = __ldg(p.tc_live_mask + (long)ks * 32 + lane);
-    int before = __popc(m);  // inclusive scan of the lanes' counts
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, before, o);
-      if (lane >= o) before += v;
-    }
-    const int* ids = tc_ids + __ldg(p.tc_live_ptr + ks) + before - __popc(m);
-    float v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const bool live = (m >> j) & 1u;
-      v[j] = live ? __ldg(hv + __ldcs(ids + __popc(m & ((1u << j) - 1u)))) : 0.f;
-    }
+__device__ __forceinline__ void pack_plan(const PackPlan& p, int block, const float* __restrict__ hv, long h,
+                                          long tc_head_bytes) {
+  if (block < p.tc_blocks) {
     constexpr uint32_t kBytes = MODE == STILE_TC_SPLIT_BF16 ? 2 * kBStage : kBStage;
-    uint4* out = reinterpret_cast<uint4*>(tc_out + h * tc_head_bytes + (long)ks * kBytes) + lane;
-    if constexpr (MODE == STILE_TC_F16) {
-      *out = make_uint4(pack_f16x2(v[0], v[1]), pack_f16x2(v[2], v[3]), pack_f16x2(v[4], v[5]), pack_f16x2(v[6], v[7]));
-    } else {
-      uint32_t hi[4];
+    const int lane = threadIdx.x & 31;
+    const int ks0 = (block * (kPackThreads / kWarp) + (threadIdx.x >> 5)) * kPackSteps;
+    unsigned m[kPackSteps];
+    const int* ids[kPackSteps];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) hi[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-      *out = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      if constexpr (MODE == STILE_TC_SPLIT_BF16) {
-        uint32_t lo[4];
+    for (int s = 0; s < kPackSteps; ++s) {
+      const bool in = ks0 + s < p.n_ks;
+      m[s] = in ? __ldg(p.mask + (long)(ks0 + s) * 32 + lane) : 0u;
+      ids[s] = p.ids + (in ? __ldg(p.ptr + ks0 + s) : 0);
+    }
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          lo[j] = pack_bf16x2(v[2 * j] - __uint_as_float(hi[j] << 16),
-                              v[2 * j + 1] - __uint_as_float(hi[j] & 0xffff0000u));
-        out[kBStage / 16] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    for (int s = 0; s < kPackSteps; ++s) {
+      int before = __popc(m[s]);  // inclusive scan of the lanes' counts
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += v;
+      }
+      ids[s] += before - __popc(m[s]);
+    }
+    float v[kPackSteps][8];
+#pragma unroll
+    for (int s = 0; s < kPackSteps; ++s) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const bool live = (m[s] >> j) & 1u;
+        v[s][j] = live ? __ldg(hv + __ldcs(ids[s] + __popc(m[s] & ((1u << j) - 1u)))) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < kPackSteps; ++s) {
+      if (ks0 + s >= p.n_ks) continue;
+      uint4* out = reinterpret_cast<uint4*>(p.tc_out + h * tc_head_bytes + (long)(ks0 + s) * kBytes) + lane;
+      const float(&x)[8] = v[s];
+      if constexpr (MODE == STILE_TC_F16) {
+        *out = make_uint4(pack_f16x2(x[0], x[1]), pack_f16x2(x[2], x[3]), pack_f16x2(x[4], x[5]),
+                          pack_f16x2(x[6], x[7]));
+      } else {
+        uint32_t hi[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) hi[j] = pack_bf16x2(x[2 * j], x[2 * j + 1]);
+        *out = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        if constexpr (MODE == STILE_TC_SPLIT_BF16) {
+          uint32_t lo[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            lo[j] = pack_bf16x2(x[2 * j] - __uint_as_float(hi[j] << 16),
+                                x[2 * j + 1] - __uint_as_float(hi[j] & 0xffff0000u));
+          out[kBStage / 16] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
       }
     }
     return;
   }
-  const long i = 4 * ((long)(blockIdx.x - tc_blocks) * kPackThreads + threadIdx.x);
-  float* __restrict__ out = ell_out + h * n_ell;
+  const long i = 4 * ((long)(block - p.tc_blocks) * kPackThreads + threadIdx.x);
+  float* __restrict__ out = p.ell_out + h * p.n_ell;
   auto value = [&](int id) { return id >= 0 ? __ldg(hv + id) : 0.f; };
-  if (i + 4 <= n_ell) {
+  if (i + 4 <= p.n_ell) {
     // the ids are 16-byte aligned; a head's values only when n_ell % 4 == 0
-    const int4 id = __ldcs(reinterpret_cast<const int4*>(ell_ids + i));
+    const int4 id = __ldcs(reinterpret_cast<const int4*>(p.ell_ids + i));
     const float4 v = make_float4(value(id.x), value(id.y), value(id.z), value(id.w));
-    if (((h * n_ell) & 3) == 0) {
+    if (((h * p.n_ell) & 3) == 0) {
       *reinterpret_cast<float4*>(out + i) = v;
     } else {
       out[i] = v.x;
@@ -1052,7 +1074,29 @@ __global__ void __launch_bounds__(kPackThreads) pack_values_kernel(SpmmArgs p, c
       out[i + 3] = v.w;
     }
   } else {
-    for (long j = i; j < n_ell; ++j) out[j] = value(__ldg(ell_ids + j));
+    for (long j = i; j < p.n_ell; ++j) out[j] = value(__ldg(p.ell_ids + j));
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kPackThreads) pack_values_kernel(PackPlan a, PackPlan b,
+                                                                   const float* __restrict__ vals, long nnz,
+                                                                   long tc_head_bytes, float* __restrict__ copy) {
+  const long h = blockIdx.y;
+  const float* __restrict__ hv = vals + h * nnz;
+  const int block = blockIdx.x;
+  if (block < a.blocks) {
+    pack_plan<MODE>(a, block, hv, h, tc_head_bytes);
+  } else if (block < a.blocks + b.blocks) {
+    pack_plan<MODE>(b, block - a.blocks, hv, h, tc_head_bytes);
+  } else {
+    // 4 values a thread, one every kPackThreads
+    const long i0 = (long)(block - a.blocks - b.blocks) * 4 * kPackThreads + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long i = i0 + k * kPackThreads;
+      if (i < nnz) copy[i] = __ldg(vals + i);
+    }
   }
 }
 
@@ -1113,20 +1157,31 @@ cudaError_t launch_amax(const float* B, long ldb, int K, int N, unsigned* amax_b
   return cudaGetLastError();
 }
 
-cudaError_t launch_pack_values(const SpmmArgs& p, const float* vals, long nnz, int heads, float* ell_out,
-                               void* tc_out, long n_ell, long tc_head_bytes, bool forward_ids, cudaStream_t st) {
-  constexpr int kWarps = kPackThreads / kWarp;
-  const int tc_blocks = (p.tc_n_ksteps + kWarps - 1) / kWarps;
-  const long ell_blocks = (n_ell + 4 * kPackThreads - 1) / (4 * kPackThreads);
-  if (tc_blocks + ell_blocks == 0 || heads == 0) return cudaSuccess;
-  const int* tc_ids = forward_ids ? p.tc_live_fid : p.tc_live_id;
-  const int* ell_ids = forward_ids ? p.ell_fid : p.ell_nnz_id;
-  const dim3 grid((unsigned)(tc_blocks + ell_blocks), (unsigned)heads);
-  auto k = p.tc_mode == STILE_TC_F16            ? pack_values_kernel<STILE_TC_F16>
-           : p.tc_mode == STILE_TC_SPLIT_BF16 ? pack_values_kernel<STILE_TC_SPLIT_BF16>
-                                              : pack_values_kernel<STILE_TC_BF16>;
-  k<<<grid, kPackThreads, 0, st>>>(p, vals, nnz, tc_ids, ell_ids, ell_out, static_cast<uint8_t*>(tc_out), n_ell,
-                                   tc_head_bytes, tc_blocks);
+PackPlan pack_of(const SpmmArgs& p, long n_ell, float* ell_out, void* tc_out, bool forward_ids) {
+  constexpr int kPer = kPackThreads / kWarp * kPackSteps;
+  PackPlan r{};
+  r.mask = p.tc_live_mask;
+  r.ptr = p.tc_live_ptr;
+  r.ids = forward_ids ? p.tc_live_fid : p.tc_live_id;
+  r.tc_out = static_cast<uint8_t*>(tc_out);
+  r.n_ks = p.tc_n_ksteps;
+  r.ell_ids = forward_ids ? p.ell_fid : p.ell_nnz_id;
+  r.ell_out = ell_out;
+  r.n_ell = n_ell;
+  r.tc_blocks = (p.tc_n_ksteps + kPer - 1) / kPer;
+  r.blocks = r.tc_blocks + (int)((n_ell + 4 * kPackThreads - 1) / (4 * kPackThreads));
+  return r;
+}
+
+cudaError_t launch_pack_values(int tc_mode, const PackPlan& a, const PackPlan& b, const float* vals, long nnz,
+                               int heads, long tc_head_bytes, float* copy, cudaStream_t st) {
+  const long copy_blocks = copy ? (nnz + 4 * kPackThreads - 1) / (4 * kPackThreads) : 0;
+  const long blocks = (long)a.blocks + b.blocks + copy_blocks;
+  if (blocks == 0 || heads == 0) return cudaSuccess;
+  auto k = tc_mode == STILE_TC_F16            ? pack_values_kernel<STILE_TC_F16>
+           : tc_mode == STILE_TC_SPLIT_BF16 ? pack_values_kernel<STILE_TC_SPLIT_BF16>
+                                            : pack_values_kernel<STILE_TC_BF16>;
+  k<<<dim3((unsigned)blocks, (unsigned)heads), kPackThreads, 0, st>>>(a, b, vals, nnz, tc_head_bytes, copy);
   return cudaGetLastError();
 }
 

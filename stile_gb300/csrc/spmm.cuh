@@ -153,11 +153,26 @@ constexpr int kChunkSteps = 32;  // most k-steps of a chunk
 constexpr int kSplitSteps = 8;   // most k-steps of a unit in the split-bf16 mode
 // unit flags: its rows are added to C; it is a chunk's first, its last unit
 constexpr int kUnitAdds = 1 << 16, kUnitFirst = 1 << 17, kUnitLast = 1 << 18;
-// the tile values of `heads` value sets (vals + h * nnz) into ell_out (+ h *
-// n_ell values) and the tensor-tile images tc_out (+ h * tc_head_bytes);
-// forward_ids: vals are in the forward operator's numbering
-cudaError_t launch_pack_values(const SpmmArgs& p, const float* vals, long nnz, int heads, float* ell_out,
-                               void* tc_out, long n_ell, long tc_head_bytes, bool forward_ids, cudaStream_t st);
+// what a value refresh reads and writes of one plan (pack_of)
+struct PackPlan {
+  const uint8_t* mask;
+  const int* ptr;
+  const int* ids;
+  uint8_t* tc_out;
+  int n_ks;
+  const int* ell_ids;
+  float* ell_out;
+  long n_ell;
+  int tc_blocks, blocks;
+};
+// forward_ids: the values are in the forward operator's numbering
+PackPlan pack_of(const SpmmArgs& p, long n_ell, float* ell_out, void* tc_out, bool forward_ids);
+// the tile values of `heads` value sets (vals + h * nnz) into the row-tile
+// values (+ h * n_ell) and tensor-tile images (+ h * tc_head_bytes) of plan a
+// and, with one head, of plan b (blocks 0: none) of the same tile mode, and
+// the values themselves into copy (NULL: none)
+cudaError_t launch_pack_values(int tc_mode, const PackPlan& a, const PackPlan& b, const float* vals, long nnz,
+                               int heads, long tc_head_bytes, float* copy, cudaStream_t st);
 // *amax_bits = bits of max |B[r][f]| over K rows x N features (atomicMax on
 // the non-negative floats' bits; *amax_bits starts at 0); an ordinary launch
 cudaError_t launch_amax(const float* B, long ldb, int K, int N, unsigned* amax_bits, cudaStream_t st);

@@ -51,7 +51,7 @@ def _padded_rows(x: torch.Tensor, ldp: int) -> torch.Tensor:
     Rows of contiguous elements go through the padding kernel (one pass over
     memory), other strides through torch."""
     rows, cols = x.shape
-    if x.stride(1) != 1 or x.requires_grad or rows * ldp >= 1 << 39:
+    if x.stride(1) != 1 or rows * ldp >= 1 << 39:
         buf = torch.zeros((rows, ldp), dtype=x.dtype, device=x.device)
         buf[:, :cols] = x
         return buf[:, :cols]
@@ -317,15 +317,19 @@ class DeviceSpmmPlan:
         _lib.check(self.lib.stile_spmm_plan_set_values(self.handle, vals.data_ptr(), _stream()),
                    "stile_spmm_plan_set_values")
 
-    def set_values_forward(self, vals: torch.Tensor):
-        """Values of A, in A's numbering, into this plan of A^T (after
-        set_transpose_ids)."""
+    def set_values_pair(self, planT: "DeviceSpmmPlan", vals: torch.Tensor) -> torch.Tensor:
+        """set_values(vals) here and set_values(vals[perm]) on planT, the plan
+        of A^T (after set_transpose_ids), in one launch; returns a copy of
+        vals."""
         _require_cuda(vals, "vals")
         vals = vals.float().contiguous()
         if vals.numel() != self.nnz:
             raise ValueError("vals must have one entry per nonzero")
-        _lib.check(self.lib.stile_spmm_plan_set_values_forward(self.handle, vals.data_ptr(), _stream()),
-                   "stile_spmm_plan_set_values_forward")
+        copy = torch.empty_like(vals)
+        _lib.check(self.lib.stile_spmm_plan_set_values_pair(self.handle, planT.handle, vals.data_ptr(),
+                                                            copy.data_ptr(), _stream()),
+                   "stile_spmm_plan_set_values_pair")
+        return copy
 
     def set_wait_policy(self, polls: int = 0, stall_test: bool = False):
         """Poll limit of the tensor-core kernel's pipeline waits (0: the
