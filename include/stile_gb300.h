@@ -316,7 +316,7 @@ int stile_spmm_backward(const StileSpmmPlan* planT, const float* dC, int64_t ldd
  * k-step's 16 columns once, against one row per nonzero), mode 2 by the
  * row runs of the entry list (fp32 on CUDA cores), mode 0 (the default at
  * upload) the row runs, which measured faster on the 232,965-node GCN
- * graph; the operator API times both once per width.  Row-tile
+ * graph and are exact to fp32; the operator API uses them.  Row-tile
  * nonzeros always take the row runs or
  * the fused ELL pass.  A bf16 B (stile_spmm_dvals_bf16) always takes the
  * row runs.  The mode is read when a call is enqueued; setting it is not

@@ -79,8 +79,8 @@ static int run_group(long entries) {
 // default of the tensor tiles' value gradients: the row runs (measured
 // faster on the GCN graph, 40.7 nonzeros per k-step: the tensor-core kernel
 // gathers fewer rows, but each CTA waits for its loads, then its MMAs, per
-// 64-feature chunk); stile_spmm_plan_set_dvals_mode(1) and the operator's
-// backward tuning select the tensor cores
+// 64-feature chunk); stile_spmm_plan_set_dvals_mode(1) selects the tensor
+// cores
 static int tcdv_auto(const StileSpmmPlan* plan) {
   (void)plan;  // one rule for every plan
   return 0;
