@@ -19,10 +19,12 @@
 // Bound by instruction issue before and by the L1 data pipe now (a strided
 // mask's neighbouring rows share their columns: two thirds of the loads hit
 // L1, and 3.1 GB of K and V rows pass the pipe): the multiply-adds are paired
-// (fma.rn.f32x2), the column ids come LPR at a time, full rows load without
-// masks and one exponential a batch serves its kU entries.  4096 tokens, 8
+// (fma.rn.f32x2), the column ids come LPR at a time, rows load without
+// predicates and one exponential a batch serves its kU entries.  4096 tokens, 8
 // heads, 64 features, strided mask (766k entries a head): 188 us with pairs of
-// entries and scalar multiply-adds, 152 us now.
+// entries and scalar multiply-adds, 152 us now; 4 heads of 41 / 80 / 127
+// features: 114 / 188 / 188 us, with predicated loads of kU entries (which
+// spilled) 128 / 182 / 205 us, now 104 / 150 / 181 us.
 #include "common.cuh"
 #include "spmm.cuh"
 
@@ -32,26 +34,25 @@ struct Feat8 {  // this lane's 8 features of a row: f .. f + 3 and f2 .. f2 + 3
   f32x2 v[4];
 };
 
-// kMask 0: the row has all 8 LPR features; 1: whole float4 up to n; 2: any n
-// (features past n are zero)
-template <int kMask>
-__device__ __forceinline__ Feat8 load8(const float* row, int f, int f2, int n) {
-  float4 a, b;
-  if constexpr (kMask == 0) {
-    a = ldg4(row + f);
-    b = ldg4(row + f2);
-  } else if constexpr (kMask == 1) {
-    a = ld4_pad(row, f, n);
-    b = ld4_pad(row, f2, n);
-  } else {
-    a = ld4_live(row, f, n);
-    b = ld4_live(row, f2, n);
-  }
-  return {{pack2(a.x, a.y), pack2(a.z, a.w), pack2(b.x, b.y), pack2(b.z, b.w)}};
+// the row's float4 at a and b (both inside the row)
+__device__ __forceinline__ Feat8 load8(const float* row, int a, int b) {
+  const float4 x = ldg4(row + a), y = ldg4(row + b);
+  return {{pack2(x.x, x.y), pack2(x.z, x.w), pack2(y.x, y.y), pack2(y.z, y.w)}};
+}
+
+// the pair with its components past the first `live` features zero
+__device__ __forceinline__ f32x2 keep2(f32x2 v, int live) {
+  const float2 x = unpack2(v);
+  return pack2(live > 0 ? x.x : 0.f, live > 1 ? x.y : 0.f);
 }
 
 constexpr int kAttThreads = 128;
 
+// kMask 0: F and Fv are 8 LPR; 1: F is a multiple of 4; 2: any F.  A lane whose
+// float4 starts past a row's features loads the row's last one instead (no
+// predicates, no zeroed registers); K's products of such a float4 are left out
+// of the score by selects (a product with a zeroed q would turn an infinite K
+// into NaN), and V's features past Fv are never stored.
 template <int LPR, int kMask>
 __global__ void __launch_bounds__(kAttThreads, 5) sparse_attention_kernel(
     int n_rows, const int* __restrict__ indptr, const int* __restrict__ indices, const float* __restrict__ Q,
@@ -67,7 +68,17 @@ __global__ void __launch_bounds__(kAttThreads, 5) sparse_attention_kernel(
   const float* Vh = V + h * v_head;
   // each load instruction of the group reads 16 LPR contiguous bytes of a row
   const int f = 4 * sl, f2 = f + 4 * LPR;
-  const Feat8 q = load8<kMask>(Q + h * q_head + r * ldq, f, f2, F);
+  const int last = (F - 1) & ~3, lastv = (Fv - 1) & ~3;
+  const int ka = kMask ? min(f, last) : f, kb = kMask ? min(f2, last) : f2;
+  const int va = kMask ? min(f, lastv) : f, vb = kMask ? min(f2, lastv) : f2;
+  Feat8 q = load8(Q + h * q_head + r * ldq, ka, kb);
+  if constexpr (kMask == 2) {
+    // q's padding; K's, which meets it, is cleared as it comes
+    q.v[0] = keep2(q.v[0], F - ka);
+    q.v[1] = keep2(q.v[1], F - ka - 2);
+    q.v[2] = keep2(q.v[2], F - kb);
+    q.v[3] = keep2(q.v[3], F - kb - 2);
+  }
   const int rb = __ldg(indptr + r), n = __ldg(indptr + r + 1) - rb;
   // this lane's entry of a batch: the halving strides' bits of its index
   int e = 0;
@@ -87,18 +98,22 @@ __global__ void __launch_bounds__(kAttThreads, 5) sparse_attention_kernel(
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
         const long c = __shfl_sync(mask, cl, b0 + u, LPR);
-        k[u] = load8<kMask>(Kh + c * ldk, f, f2, F);
-        // features past Fv are never stored
-        v[u] = load8<(kMask == 0 ? 0 : 1)>(Vh + c * ldv, f, f2, Fv);
+        k[u] = load8(Kh + c * ldk, ka, kb);
+        v[u] = load8(Vh + c * ldv, va, vb);
       }
       float s[kU];
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
-        f32x2 d = mul2(q.v[0], k[u].v[0]);
-#pragma unroll
-        for (int w = 1; w < 4; ++w) d = fma2(q.v[w], k[u].v[w], d);
-        const float2 p = unpack2(d);
-        s[u] = p.x + p.y;
+        if constexpr (kMask == 2) {
+          k[u].v[0] = keep2(k[u].v[0], F - ka);
+          k[u].v[1] = keep2(k[u].v[1], F - ka - 2);
+          k[u].v[2] = keep2(k[u].v[2], F - kb);
+          k[u].v[3] = keep2(k[u].v[3], F - kb - 2);
+        }
+        const f32x2 da = fma2(q.v[1], k[u].v[1], mul2(q.v[0], k[u].v[0]));
+        const f32x2 d = fma2(q.v[3], k[u].v[3], fma2(q.v[2], k[u].v[2], da));
+        const float2 p = unpack2(kMask == 0 || f2 < F ? d : da);
+        s[u] = kMask == 0 || f < F ? p.x + p.y : 0.f;
       }
       // transposing butterfly: this lane keeps entry e's score
 #pragma unroll
