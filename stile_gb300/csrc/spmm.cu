@@ -1474,8 +1474,13 @@ cudaError_t launch_ell(const SpmmArgs& args, cudaStream_t st) {
   // wider rows that are no multiple of 128: 256 features a pass (two float4 a
   // lane) where that covers no more than passes of 128 do (one float4): N = 150
   // on the 50,000-node graph 133 -> 121 us; N = 300 on the 169k-node graph would
-  // go from 179 to 186
-  if ((p.N + 255) / 256 * 2 == (p.N + 127) / 128) return EllNarrowLaunch<32>::run(p, st);
+  // go from 179 to 186.  Not where the passes of 128, a block each, leave SMs
+  // idle: a block then lasts as long as its longest group times its features
+  // (N = 150, 21,198 entries: 5.8 against 7.5 us; 47,232 entries fill the
+  // device: 8.7 against 7.9).
+  const long blocks = (p.ell_n_groups + 7L) / 8 * ((p.N + 127) / 128);
+  if ((p.N + 255) / 256 * 2 == (p.N + 127) / 128 && blocks >= 5L * device_sm_count())
+    return EllNarrowLaunch<32>::run(p, st);
   return EllLaunch<32>::run(p, st);
 }
 
