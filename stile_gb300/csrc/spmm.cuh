@@ -150,7 +150,7 @@ cudaError_t launch_tc_dvals(const SpmmArgs& p, const float* X, long ldx, const f
                             cudaStream_t st);
 constexpr int kTcDvUnit = 8;  // k-steps per unit of the tensor-tile value-gradient kernel
 constexpr int kChunkSteps = 32;  // most k-steps of a chunk
-constexpr int kSplitSteps = 8;   // most k-steps of a unit in the split-bf16 mode
+constexpr int kSplitSteps = 4;   // most k-steps of a unit in the split-bf16 mode
 // unit flags: its rows are added to C; it is a chunk's first, its last unit
 constexpr int kUnitAdds = 1 << 16, kUnitFirst = 1 << 17, kUnitLast = 1 << 18;
 // what a value refresh reads and writes of one plan (pack_of)
