@@ -353,6 +353,11 @@ int stile_sddmm_plan_error_flag(StileSddmmPlan* plan, void* stream, int32_t* fla
  * threads. */
 int stile_spmm_plan_set_wait_policy(StileSpmmPlan* plan, int32_t polls, int32_t stall_test);
 
+/* The same for the block kernel of an SDDMM plan, whose one wait is for a
+ * unit's MMAs: when it gives up, the scores of the unit and of the units its
+ * CTA has not begun are 0 and the error flag is set. */
+int stile_sddmm_plan_set_wait_policy(StileSddmmPlan* plan, int32_t polls, int32_t stall_test);
+
 /* Tensor-core layout self-check (no counterpart in the reference): runs one
  * tcgen05.mma (M=128, N=16; kind = 0: kind::f16, K=16; kind = 1:
  * kind::tf32, K=8; kind = 2: kind::f8f6f4, K=32; fp32 accumulate) on two 16 KB shared-memory images copied

@@ -1023,6 +1023,15 @@ int stile_spmm_plan_set_wait_policy(StileSpmmPlan* plan, int32_t polls, int32_t 
   return STILE_OK;
 }
 
+int stile_sddmm_plan_set_wait_policy(StileSddmmPlan* plan, int32_t polls, int32_t stall_test) {
+  if (!plan) return fail(STILE_E_INVALID, "null plan");
+  if (stall_test && polls <= 0)
+    return fail(STILE_E_INVALID, "a stall test needs a poll limit (the default wait lasts seconds)");
+  plan->args.poll_limit = polls > 0 ? (uint32_t)polls : 0u;
+  plan->args.stall_test = stall_test ? 1 : 0;
+  return STILE_OK;
+}
+
 int stile_sparse_attention(int32_t n_rows, const int32_t* indptr, const int32_t* indices, const float* Q,
                            const float* K, const float* V, int64_t ldq, int64_t ldk, int64_t ldv,
                            int64_t q_head_stride, int64_t k_head_stride, int64_t v_head_stride, float* out,

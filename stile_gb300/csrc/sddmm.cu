@@ -431,8 +431,8 @@ cudaError_t launch_sddmm_runs(int n_groups, const int* gptr, const int* grow, co
 // reads each warp's 32 Y rows from TMEM, stages the diagonal blocks in shared
 // memory and writes only the blocks' live entries (indicesDense), 4 entries of
 // the unit's contiguous list in flight per thread.  The wait for the MMAs is
-// bounded; a wait that runs out sets the error flag and skips the unit's
-// output.
+// bounded; a wait that runs out sets the error flag and gives the unit's and
+// the CTA's later entries zeros.
 // Bound by latency (a mask gives each CTA a unit or two): one thread per row
 // walking its 64 features, and the blocks' entry lists walked one after
 // another, took 17 us for the 1,703 blocks of a 100,000-row mask at F = 64.
@@ -449,8 +449,9 @@ struct BlkCfg {
   static constexpr uint32_t kBytes = 1024 + kImgs * kBlkImg + kDBytes + 64;
 };
 
+// (without a block count the compiler settled on 64 registers with spills in fp32)
 template <bool kB16>
-__global__ void __launch_bounds__(kBlkThreads) sddmm_block_tc_kernel(SddmmArgs p, int n_units, int lazy_wait) {
+__global__ void __launch_bounds__(kBlkThreads, kB16 ? 4 : 3) sddmm_block_tc_kernel(SddmmArgs p, int n_units, int lazy_wait) {
   using Cfg = BlkCfg<kB16>;
   // lazy_wait: launched dependent on the 1D kernel of the same call, which
   // writes other entries; only the end of this grid implies that one's end
@@ -461,11 +462,12 @@ __global__ void __launch_bounds__(kBlkThreads) sddmm_block_tc_kernel(SddmmArgs p
   const uint32_t yhi = base, xhi = base + kBlkImg, ylo = base + 2 * kBlkImg, xlo = base + 3 * kBlkImg;
   const uint32_t dst = base + Cfg::kImgs * kBlkImg;
   float* dstage = reinterpret_cast<float*>(smem_raw + (dst - smem_u32(smem_raw)));
-  const uint32_t bar = dst + Cfg::kDBytes, tmem_slot = bar + 8;
+  const uint32_t bar = dst + Cfg::kDBytes, tmem_slot = bar + 8, stall = bar + 16;
   __shared__ int s_ptr[kBlkUnit + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     mbar_init(bar, 1);
+    mbar_init(stall, 1);
     fence_mbar_init();
   }
   if (warp == 0) {
@@ -486,8 +488,10 @@ __global__ void __launch_bounds__(kBlkThreads) sddmm_block_tc_kernel(SddmmArgs p
   const int F = p.F;
   uint32_t phase = 0;
   bool ok = true;
+  const uint32_t polls = p.poll_limit ? p.poll_limit : kDefaultPolls;
+  int u = blockIdx.x;
 #pragma unroll 1
-  for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+  for (; u < n_units; u += gridDim.x) {
     const int b0 = u * kBlkUnit;
     const int nb = min(kBlkUnit, p.n_blk - b0);
     if (tid <= nb) s_ptr[tid] = __ldg(p.blk_indptr + b0 + tid);
@@ -550,7 +554,10 @@ __global__ void __launch_bounds__(kBlkThreads) sddmm_block_tc_kernel(SddmmArgs p
         umma_commit(bar);
       }
       // the MMAs read the images: nobody rewrites them, or reads TMEM, first
-      const bool done = __syncthreads_and(tid == 0 ? mbar_wait_bounded(bar, phase) : true) != 0;
+      // (failure-detection test: nothing arrives on `stall`)
+      bool got = true;
+      if (tid == 0) got = (!p.stall_test || mbar_wait_bounded(stall, 0u, polls)) && mbar_wait_bounded(bar, phase, polls);
+      const bool done = __syncthreads_and(got) != 0;
       phase ^= 1u;
       if (!done) {
         ok = false;
@@ -600,6 +607,14 @@ __global__ void __launch_bounds__(kBlkThreads) sddmm_block_tc_kernel(SddmmArgs p
       }
     }
     __syncthreads();
+  }
+  // a wait gave up: the scores of the unit and of this CTA's later ones are 0
+  // (the caller's buffer may hold anything)
+  if (!ok) {
+    for (; u < n_units; u += gridDim.x) {
+      const int e1 = __ldg(p.blk_indptr + min((u + 1) * kBlkUnit, p.n_blk));
+      for (int e = __ldg(p.blk_indptr + u * kBlkUnit) + tid; e < e1; e += kBlkThreads) p.out[__ldg(p.blk_out + e)] = 0.f;
+    }
   }
   if (lazy_wait) griddep_wait();
   if (!ok && tid == 0 && p.err_flag) atomicOr(p.err_flag, 1);

@@ -205,8 +205,12 @@ struct SddmmArgs {
   const int* blk_dense_pos;
   const int* blk_out;
   int disjoint;  // no entry is in a 1D and in a block tile
-  // device error flag (the block kernel's bounded MMA wait gave up)
+  // device error flag (the block kernel's bounded MMA wait gave up), the poll
+  // limit of that wait (0: the default) and the failure-detection test, in
+  // which it waits on a barrier that nothing arrives on
   int* err_flag;
+  uint32_t poll_limit;
+  int stall_test;
 };
 
 cudaError_t launch_sddmm(const SddmmArgs& p, cudaStream_t st);

@@ -374,11 +374,18 @@ class DeviceSddmmPlan:
         _lib.check(self.lib.stile_sddmm_plan_upload(ctypes.byref(h), ctypes.byref(handle)),
                    "stile_sddmm_plan_upload")
         self.handle = handle
-        # every entry is in a tile: a run writes all of its output
+        # every entry is in a tile: a run writes all of its output (zeros where
+        # the block kernel's wait gives up)
         hit = np.zeros(dev.nnz, dtype=bool)
         hit[dev.remap] = True
         hit[dev.blk_out] = True
         self._cover_all = bool(hit.all())
+
+    def set_wait_policy(self, polls: int = 0, stall_test: bool = False):
+        """Poll limit of the block kernel's wait for its MMAs (0: the default)
+        and the failure-detection stall test (stile_sddmm_plan_set_wait_policy)."""
+        _lib.check(self.lib.stile_sddmm_plan_set_wait_policy(self.handle, int(polls), 1 if stall_test else 0),
+                   "stile_sddmm_plan_set_wait_policy")
 
     def error_flag(self) -> int:
         f = ctypes.c_int32(0)
