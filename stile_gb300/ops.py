@@ -214,7 +214,6 @@ class DeviceSpmmPlan:
                    "stile_spmm_plan_upload")
         self.handle = handle
         self._dvals_cover_all = _tiles_cover_every_nonzero(dev)
-        self._dvals_mode = 0  # as set_dvals_mode set it last (0: as uploaded)
         # tensor tiles with nonzero ids: their value gradients can run on the
         # tensor cores (stile_spmm_plan_set_dvals_mode)
         self.has_tensor_tiles = len(dev.tc_cols) > 0 and len(dev.tc_nnz_id) > 0
@@ -341,10 +340,7 @@ class DeviceSpmmPlan:
     def set_dvals_mode(self, mode: int):
         """Value gradients of the tensor-tile nonzeros: 0 automatic, 1 on the
         tensor cores, 2 by the row runs (stile_spmm_plan_set_dvals_mode)."""
-        if int(mode) == self._dvals_mode:
-            return
         _lib.check(self.lib.stile_spmm_plan_set_dvals_mode(self.handle, int(mode)), "stile_spmm_plan_set_dvals_mode")
-        self._dvals_mode = int(mode)
 
     def error_flag(self) -> int:
         f = ctypes.c_int32(0)
