@@ -159,10 +159,12 @@ class SpmmOperator:
 
     @property
     def _vals(self):
-        """The values last loaded, in this operator's CSR order, or None."""
+        """The values last loaded, in this operator's CSR order, or None.  Those
+        of a transposed operator are permuted anew on every call: a graph that
+        loads values writes the operator's copy on each replay."""
         if isinstance(self._vals_src, tuple):
             vals, perm = self._vals_src
-            self._vals_src = vals[perm]
+            return vals[perm]
         return self._vals_src
 
     def _plain_ops(self):
