@@ -24,3 +24,13 @@ def test_transposed_values_follow_a_replayed_graph():
         graph.replay()
         assert torch.equal(opT._vals, vals[perm])
         assert torch.equal(op._vals, vals)
+
+
+@pytest.mark.parametrize("shape", [(1, -1), (-1, 1)], ids=["row", "column"])
+def test_values_of_another_shape(shape):
+    A = syn.power_law_rows(300, 200, min_len=2, max_len=40, seed=5)
+    op = SpmmOperator(A, 32, PlanConfig())
+    opT, perm = op.transposed
+    vals = torch.arange(A.nnz, dtype=torch.float32, device="cuda")
+    op.set_values(vals.reshape(shape))
+    assert torch.equal(op._vals, vals) and torch.equal(opT._vals, vals[perm])
