@@ -49,9 +49,9 @@ def dense_operand(x: torch.Tensor, name="B"):
 def _padded_rows(x: torch.Tensor, ldp: int) -> torch.Tensor:
     """x [rows, cols] as a view of a [rows, ldp] buffer whose padding is zero.
     Rows of contiguous elements go through the padding kernel (one pass over
-    memory), other strides through torch."""
+    memory), other strides and views that negate on reading through torch."""
     rows, cols = x.shape
-    if x.stride(1) != 1 or rows * ldp >= 1 << 39:
+    if x.stride(1) != 1 or x.is_neg() or rows * ldp >= 1 << 39:
         buf = torch.zeros((rows, ldp), dtype=x.dtype, device=x.device)
         buf[:, :cols] = x
         return buf[:, :cols]
