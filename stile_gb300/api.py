@@ -299,7 +299,9 @@ class SpmmOperator:
         """Load new values for A's pattern (``vals`` [nnz], CSR order) into
         the plan, and into the transposed plan when it exists; a transposed
         plan built later starts from these values too."""
-        vals = vals.detach().float().reshape(-1).contiguous()
+        vals = vals.detach().float().contiguous()
+        if vals.dim() != 1:
+            vals = vals.reshape(-1)
         if vals.numel() != self.nnz:
             raise ValueError("vals must have one entry per nonzero")
         if self._plain is not None:
