@@ -328,9 +328,9 @@ int stile_spmm_plan_set_dvals_mode(StileSpmmPlan* plan, int32_t mode);
  * Used when A's values change between calls (training the values). */
 int stile_spmm_plan_set_values(StileSpmmPlan* plan, const float* vals, void* stream);
 
-/* The same for the plan and, in the same launch, for the plan of A^T (after
- * stile_spmm_plan_set_transpose_ids: from the forward's values, no permuted
- * copy of them is made), and vals into copy[nnz] (NULL: no copy).  The
+/* The same for the plan and, in the same launch, for the plan of A^T (NULL:
+ * none; after stile_spmm_plan_set_transpose_ids: from the forward's values, no
+ * permuted copy of them is made), and vals into copy[nnz] (NULL: no copy).  The
  * plans' tensor tiles must have one mode (else STILE_E_UNSUPPORTED). */
 int stile_spmm_plan_set_values_pair(StileSpmmPlan* plan, StileSpmmPlan* planT, const float* vals, float* copy,
                                     void* stream);

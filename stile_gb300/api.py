@@ -317,8 +317,7 @@ class SpmmOperator:
                 self._vals_src = self.handle.set_values_pair(opT.handle, vals)
                 opT._vals_src = (self._vals_src, perm_t)
                 return
-        self.handle.set_values(vals)
-        self._vals_src = vals.clone()
+        self._vals_src = self.handle.set_values_pair(None, vals)
         if self._transposed is not None:
             opT.set_values(self._vals_src[perm_t])
 

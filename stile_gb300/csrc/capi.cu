@@ -986,16 +986,21 @@ int stile_spmm_plan_set_values(StileSpmmPlan* plan, const float* vals, void* str
 int stile_spmm_plan_set_values_pair(StileSpmmPlan* plan, StileSpmmPlan* planT, const float* vals, float* copy,
                                     void* stream) {
   stile::begin_call();
-  if (!plan || !planT || !vals) return fail(STILE_E_INVALID, "null argument");
-  if (planT->nnz != plan->nnz) return fail(STILE_E_INVALID, "the plans must have the same nonzeros");
-  // a plan without tensor tiles takes either mode
-  if (plan->args.tc_n_ksteps && planT->args.tc_n_ksteps && plan->args.tc_mode != planT->args.tc_mode)
-    return fail(STILE_E_UNSUPPORTED, "the plans must have the same tensor-tile mode");
+  if (!plan || !vals) return fail(STILE_E_INVALID, "null argument");
   if (int rc = check_refresh(plan, false)) return rc;
-  if (int rc = check_refresh(planT, true)) return rc;
-  const int mode = plan->args.tc_n_ksteps ? plan->args.tc_mode : planT->args.tc_mode;
-  cudaError_t e = stile::launch_pack_values(mode, own_values(plan, false), own_values(planT, true), vals, plan->nnz, 1,
-                                            0, copy, static_cast<cudaStream_t>(stream));
+  int mode = plan->args.tc_mode;
+  stile::PackPlan second{};
+  if (planT) {
+    if (planT->nnz != plan->nnz) return fail(STILE_E_INVALID, "the plans must have the same nonzeros");
+    // a plan without tensor tiles takes either mode
+    if (plan->args.tc_n_ksteps && planT->args.tc_n_ksteps && mode != planT->args.tc_mode)
+      return fail(STILE_E_UNSUPPORTED, "the plans must have the same tensor-tile mode");
+    if (int rc = check_refresh(planT, true)) return rc;
+    if (!plan->args.tc_n_ksteps) mode = planT->args.tc_mode;
+    second = own_values(planT, true);
+  }
+  cudaError_t e = stile::launch_pack_values(mode, own_values(plan, false), second, vals, plan->nnz, 1, 0, copy,
+                                            static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "value re-pack launch");
   g_launches++;
   return STILE_OK;

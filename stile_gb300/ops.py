@@ -316,17 +316,17 @@ class DeviceSpmmPlan:
         _lib.check(self.lib.stile_spmm_plan_set_values(self.handle, vals.data_ptr(), _stream()),
                    "stile_spmm_plan_set_values")
 
-    def set_values_pair(self, planT: "DeviceSpmmPlan", vals: torch.Tensor) -> torch.Tensor:
+    def set_values_pair(self, planT: "DeviceSpmmPlan | None", vals: torch.Tensor) -> torch.Tensor:
         """set_values(vals) here and set_values(vals[perm]) on planT, the plan
-        of A^T (after set_transpose_ids), in one launch; returns a copy of
-        vals."""
+        of A^T (after set_transpose_ids; None: no such plan), in one launch;
+        returns a copy of vals."""
         _require_cuda(vals, "vals")
         vals = vals.float().contiguous()
         if vals.numel() != self.nnz:
             raise ValueError("vals must have one entry per nonzero")
         copy = torch.empty_like(vals)
-        _lib.check(self.lib.stile_spmm_plan_set_values_pair(self.handle, planT.handle, vals.data_ptr(),
-                                                            copy.data_ptr(), _stream()),
+        _lib.check(self.lib.stile_spmm_plan_set_values_pair(self.handle, planT.handle if planT else None,
+                                                            vals.data_ptr(), copy.data_ptr(), _stream()),
                    "stile_spmm_plan_set_values_pair")
         return copy
 
