@@ -210,7 +210,6 @@ constexpr int kAccBufs = 8;                        // accumulators of 16 TMEM co
 // is in unit y has written every unit below y - kLag, so the MMA of unit y or
 // an earlier one finds its accumulator read
 constexpr int kLag = 4;
-static_assert(kLag < kAccBufs, "the MMA warp waits for accumulators that every warp has passed");
 
 // Split-bf16 (fp32-level accuracy) keeps hi and lo images of both operands:
 // A = hi(B rows) | lo(B rows), values = hi | lo, and issues three MMAs per
@@ -242,6 +241,10 @@ struct TcCfg {
   // full and empty per slot, full and empty per accumulator, drain, TMEM address
   static constexpr uint32_t kBytes = 1024 + kBars + 16 * kTcWarps * kNs + 16 * kAccBufs + 16;
   static_assert(kSpw == 1 || kSpw == 2 || kSpw == 4, "a stage is 16 loads");
+  // a stage holds k-steps of up to kSpw units: a warp that waits with a stage
+  // which begins in unit y has not written unit y - kLag, and the MMA warp may
+  // wait for that stage in unit y + kSpw - 1
+  static_assert(kLag + kSpw - 1 < kAccBufs, "the MMA warp waits for accumulators that every warp has passed");
   static_assert(!(kIn16 && MODE != STILE_TC_BF16), "a bf16 B feeds bf16 MMAs");
   static_assert(MODE != STILE_TC_FP8 || kSpw == 1, "fp8 converts whole 16-row stages");
   static_assert(kTcCtas * (kBytes + 1024) <= 228 * 1024, "resident CTAs");
