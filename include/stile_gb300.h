@@ -371,7 +371,7 @@ int stile_debug_umma_probe(const void* a_img, const void* b_img, const uint32_t*
 /* Dense operand rows as the kernels read them: `rows` rows of `cols` elements
  * of 2 or 4 bytes, src_ld elements apart (any stride and alignment of whole
  * elements), into rows of dst_ld elements (dst_ld * elem_bytes a multiple of
- * 16, dst 16-byte aligned); the elements past cols become 0. */
+ * 16 and dst_ld < 2^31, dst 16-byte aligned); the elements past cols become 0. */
 int stile_pad_rows(const void* src, int64_t rows, int32_t cols, int64_t src_ld,
                    int32_t elem_bytes, void* dst, int64_t dst_ld, void* stream);
 

@@ -1085,6 +1085,8 @@ int stile_pad_rows(const void* src, int64_t rows, int32_t cols, int64_t src_ld, 
   if (!src || !dst) return fail(STILE_E_INVALID, "null argument");
   if (dst_ld < cols || (dst_ld * elem_bytes) % 16 != 0 || (reinterpret_cast<uintptr_t>(dst) & 15) != 0)
     return fail(STILE_E_INVALID, "dst: rows of whole 16-byte vectors, 16-byte aligned");
+  // (the kernel counts a row's elements in 32 bits)
+  if (dst_ld > INT32_MAX) return fail(STILE_E_UNSUPPORTED, "dst: rows of 2^31 elements or more");
   if ((reinterpret_cast<uintptr_t>(src) & (elem_bytes - 1)) != 0) return fail(STILE_E_INVALID, "src: misaligned elements");
   if (rows > (INT64_C(1) << 38) / (dst_ld * elem_bytes / 16))
     return fail(STILE_E_UNSUPPORTED, "more rows than one launch covers");

@@ -51,7 +51,7 @@ def _padded_rows(x: torch.Tensor, ldp: int) -> torch.Tensor:
     Rows of contiguous elements go through the padding kernel (one pass over
     memory), other strides and views that negate on reading through torch."""
     rows, cols = x.shape
-    if x.stride(1) != 1 or x.is_neg() or rows * ldp >= 1 << 39:
+    if x.stride(1) != 1 or x.is_neg() or rows * ldp >= 1 << 39 or ldp >= 1 << 31:
         buf = torch.zeros((rows, ldp), dtype=x.dtype, device=x.device)
         buf[:, :cols] = x
         return buf[:, :cols]
