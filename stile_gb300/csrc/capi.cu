@@ -59,7 +59,6 @@ struct StileSpmmPlan {
   long nnz = 0, ell_n_slots = 0;
   int n_zero_rows = 0;
   const int* zero_rows = nullptr;
-  long n_tc_dv = 0;  // tensor-tile nonzeros of the value-gradient list
   long n_tc_live = 0;  // live elements of the tensor-tile value images
   bool ids_set = false;  // set_transpose_ids has run
 };
@@ -593,6 +592,7 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
   a.dv_id = (const int*)P(i_dvi);
   a.dv_n_groups = (int)dv_grow.size();
   a.dv_n_groups_tc = dv_groups_tc;
+  a.dv_n_tc = n_tc_dv;
   a.dv_gptr = (const int*)P(i_dvgp);
   a.dv_grow = (const int*)P(i_dvgr);
   a.tc_unit_meta = (const int*)P(i_unm);
@@ -606,7 +606,6 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
   a.tcdv_unit_ks = (const int*)P(i_uks);
   a.tcdv_unit_meta = (const int*)P(i_umeta);
   a.tcdv_id = a.tc_nnz_id;  // the plan's own numbering until set_transpose_ids
-  plan->n_tc_dv = n_tc_dv;
   a.tcdv_use = tcdv_auto(plan);  // the row runs until the caller selects the tensor cores
   *out = plan;
   return STILE_OK;
@@ -879,7 +878,8 @@ static int tc_dvals(const stile::SpmmArgs& a, const int* run_ids, const float* X
     g_launches += (a.tcdv_n_units > 0);
     const int n = a.dv_n_groups - a.dv_n_groups_tc;
     if (ell && n > 0) {
-      e = stile::launch_sddmm_runs(n, a.dv_gptr + a.dv_n_groups_tc, a.dv_grow + a.dv_n_groups_tc, a.dv_col, run_ids,
+      e = stile::launch_sddmm_runs(n, a.dv_n - a.dv_n_tc, a.dv_gptr + a.dv_n_groups_tc,
+                                   a.dv_grow + a.dv_n_groups_tc, a.dv_col, run_ids,
                                    X, false, ldx, Y, false, ldy, out, N, st);
       if (e != cudaSuccess) return cuda_fail(e, "dvals launch");
       g_launches++;
@@ -887,7 +887,8 @@ static int tc_dvals(const stile::SpmmArgs& a, const int* run_ids, const float* X
     return STILE_OK;
   }
   const int n = ell ? a.dv_n_groups : a.dv_n_groups_tc;
-  e = stile::launch_sddmm_runs(n, a.dv_gptr, a.dv_grow, a.dv_col, run_ids, X, false, ldx, Y, false, ldy, out, N, st);
+  e = stile::launch_sddmm_runs(n, ell ? a.dv_n : a.dv_n_tc, a.dv_gptr, a.dv_grow, a.dv_col, run_ids, X, false, ldx, Y,
+                               false, ldy, out, N, st);
   if (e != cudaSuccess) return cuda_fail(e, "dvals launch");
   g_launches += (n > 0);
   return STILE_OK;

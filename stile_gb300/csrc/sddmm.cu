@@ -359,9 +359,9 @@ __global__ void __launch_bounds__(256, MINB) sddmm_run_kernel(int n_groups, cons
 }
 
 template <int L, bool kYb, bool kXb = false>
-static cudaError_t launch_runs_t(int grid, bool one, bool full, cudaStream_t st, int n_groups, const int* gptr,
-                                 const int* grow, const int* cols, const int* outs, const void* X, long ldx,
-                                 const void* Y, long ldy, float* out, int F) {
+static cudaError_t launch_runs_t(int grid, bool one, bool full, bool few, cudaStream_t st, int n_groups,
+                                 const int* gptr, const int* grow, const int* cols, const int* outs, const void* X,
+                                 long ldx, const void* Y, long ldy, float* out, int F) {
   // narrow rows (8 lanes or fewer: 64 features or fewer) keep 4 Y rows in
   // flight per group at 5 blocks per SM: a narrow row is few bytes, and the
   // gathers are bound by the bytes in flight
@@ -379,14 +379,16 @@ static cudaError_t launch_runs_t(int grid, bool one, bool full, cudaStream_t st,
   // several passes (or longer rows): 4 rows and the X slice in flight per pass
   // (2 rows at 6 blocks: 264 against 206 us at F = 4096 on a 768 x 3072
   // weight); the addresses are formed once per entry and pass, and the 64-bit
-  // product was the faster one (206 against 215 us)
+  // product was the faster one (206 against 215 us).  Short groups: 2 rows at 6
+  // blocks, which gather less past a group's end and start more groups at once.
+  if (few) return STILE_RUN_KERNEL(2, 6, false, false, kRow64);
   return STILE_RUN_KERNEL(4, 4, false, false, kRow64);
 #undef STILE_RUN_KERNEL
 }
 
-cudaError_t launch_sddmm_runs(int n_groups, const int* gptr, const int* grow, const int* cols, const int* outs,
-                              const void* X, bool x_bf16, long ldx, const void* Y, bool y_bf16, long ldy, float* out,
-                              int F, cudaStream_t st) {
+cudaError_t launch_sddmm_runs(int n_groups, long n_entries, const int* gptr, const int* grow, const int* cols,
+                              const int* outs, const void* X, bool x_bf16, long ldx, const void* Y, bool y_bf16,
+                              long ldy, float* out, int F, cudaStream_t st) {
   if (n_groups <= 0) return cudaSuccess;
   if (x_bf16 && !y_bf16) return cudaErrorNotSupported;  // no caller has a bf16 X with an fp32 Y
   // lanes per run: 8 features per lane (two float4, or one bf16 load);
@@ -399,7 +401,14 @@ cudaError_t launch_sddmm_runs(int n_groups, const int* gptr, const int* grow, co
   }
   const bool one = F <= 8 * lpr, full = F == 8 * lpr;
   const int grid = (int)(((long)n_groups * lpr + 255) / 256);
-#define STILE_RUNS_ARGS grid, one, full, st, n_groups, gptr, grow, cols, outs, X, ldx, Y, ldy, out, F
+  // Short groups, for rows of several passes: under 3 entries on average, or
+  // under 11 with more groups than the device keeps resident (48 warps per SM).
+  // 3M entries of 256 bf16 features in rows of 2 / 6 / 10 / 12 / 24: 333 / 199 /
+  // 175 / 171 / 165 us with 2 rows in flight, 503 / 242 / 191 / 165 / 145 with 4;
+  // 30,000 entries in rows of 4 / 8: 5.1 / 6.6 against 4.7 / 5.4.
+  const bool few = n_entries < 3L * n_groups ||
+                   (n_entries < 11L * n_groups && (long)n_groups * lpr > 48L * 32 * device_sm_count());
+#define STILE_RUNS_ARGS grid, one, full, few, st, n_groups, gptr, grow, cols, outs, X, ldx, Y, ldy, out, F
   switch (lpr) {
     case 4:
       return x_bf16 ? launch_runs_t<4, true, true>(STILE_RUNS_ARGS)
@@ -652,7 +661,7 @@ cudaError_t launch_sddmm(const SddmmArgs& p, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   if (!p.disjoint && (e = launch_blocks(p, false, st)) != cudaSuccess) return e;
   // the flattened entries come in runs of one row (cut at upload)
-  e = launch_sddmm_runs(p.n_runs, p.run_ptr, p.run_row, p.j_idx, p.remap, p.X, p.xy_bf16, p.ldx, p.Y, p.xy_bf16, p.ldy,
+  e = launch_sddmm_runs(p.n_runs, p.n_1d, p.run_ptr, p.run_row, p.j_idx, p.remap, p.X, p.xy_bf16, p.ldx, p.Y, p.xy_bf16, p.ldy,
                         p.out, p.F, st);
   if (e != cudaSuccess || !p.disjoint) return e;
   return launch_blocks(p, p.n_runs > 0, st);

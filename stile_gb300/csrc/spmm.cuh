@@ -98,7 +98,8 @@ struct SpmmArgs {
   // fused backward (this plan is the transposed operator's): the ELL pass
   // that computes dB = A^T dC also writes dvals[id] = <dC[col], dvx[row]>
   // for its entries, id from ell_fid (dvx: the forward's dense operand), and
-  // the run list's tensor-core prefix (dv_n_groups_tc groups) gives the rest
+  // the run list's tensor-core prefix (dv_n_groups_tc groups of dv_n_tc
+  // entries) gives the rest
   // with ids dvp_id; ids in the forward operator's nonzero numbering (set by
   // set_transpose_ids)
   const float* dvx;
@@ -106,6 +107,7 @@ struct SpmmArgs {
   float* dv_out;
   const int* dvp_id;
   int dv_n_groups_tc;
+  long dv_n_tc;
   // value gradients of the tensor-tile nonzeros on the tensor cores: units
   // of up to 8 k-steps of one chunk (tcdv_unit_ks: first k-step in schedule
   // order; tcdv_unit_meta: item * 8 + k-steps - 1); tcdv_id: the k-steps'
@@ -218,11 +220,12 @@ cudaError_t launch_csr_row_softmax(int M, const int* indptr, long nnz, const flo
                                    int batch, cudaStream_t st);
 cudaError_t launch_sddmm_list(long n, const int* rows, const int* cols, const int* outs, const void* X, bool x_bf16,
                               long ldx, const void* Y, bool y_bf16, long ldy, float* out, int F, cudaStream_t st);
-// row-run SDDMM: group g is entries [gptr[g], gptr[g+1]) of row grow[g]
+// row-run SDDMM: group g is entries [gptr[g], gptr[g+1]) of row grow[g];
+// n_entries: of all groups
 constexpr int kRunGroup = 64;  // entries per run group at most
-cudaError_t launch_sddmm_runs(int n_groups, const int* gptr, const int* grow, const int* cols, const int* outs,
-                              const void* X, bool x_bf16, long ldx, const void* Y, bool y_bf16, long ldy, float* out,
-                              int F, cudaStream_t st);
+cudaError_t launch_sddmm_runs(int n_groups, long n_entries, const int* gptr, const int* grow, const int* cols,
+                              const int* outs, const void* X, bool x_bf16, long ldx, const void* Y, bool y_bf16,
+                              long ldy, float* out, int F, cudaStream_t st);
 
 cudaError_t launch_sparse_attention(int n_rows, const int* indptr, const int* indices, const float* Q,
                                     const float* K, const float* V, long ldq, long ldk, long ldv, long q_head,
