@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <numeric>
 #include <queue>
 #include <string>
 #include <vector>
@@ -471,10 +472,14 @@ int stile_spmm_plan_upload(const StileSpmmPlanHost* h, StileSpmmPlan** out) {
   if (ndv > INT32_MAX) return fail(STILE_E_INVALID, "too many nonzeros for the value-gradient list");
   // units of the tensor-tile value-gradient kernel: up to kTcDvUnit k-steps
   // of one chunk (chunks are in schedule order here, their k-steps
-  // contiguous)
-  std::vector<int32_t> u_ks, u_meta;
+  // contiguous), the items in order: neighbouring items gather the same
+  // columns (169,343-node graph at 192 features: 158 us in the order of a
+  // schedule over 608 CTAs, 163 in that over 456, 146 in item order)
+  std::vector<int32_t> u_ks, u_meta, by_item((size_t)nck);
+  std::iota(by_item.begin(), by_item.end(), 0);
+  std::stable_sort(by_item.begin(), by_item.end(), [&](int32_t x, int32_t y) { return ck_item[x] < ck_item[y]; });
   if (h->tc_nnz_id && h->tc_n_items > 0)
-    for (long c = 0; c < nck; ++c)
+    for (const int32_t c : by_item)
       for (int o = 0; o < ck_nk[c]; o += stile::kTcDvUnit) {
         u_ks.push_back(ck_kbeg[c] + o);
         u_meta.push_back(ck_item[c] * stile::kTcDvUnit + std::min(stile::kTcDvUnit, ck_nk[c] - o) - 1);
