@@ -64,8 +64,9 @@ struct StileSpmmPlan {
   bool ids_set = false;  // set_transpose_ids has run
 };
 
-// Most entries of a run group: kRunGroup, or 32, 16 or 8 where that gives fewer
-// than two groups per warp the device keeps resident (48 per SM).  A group
+// Most entries of a run group: the largest of kRunGroup, 32 and 16 that the
+// entries would fill 96 times per SM, else 8 (a warp takes 2 to 8 groups at
+// once, an SM 32 to 48 warps: one to a few rounds of full groups).  A group
 // gathers its rows a few at a time, so a small list is bound by its longest
 // group: 430,000 entries at 100 bf16 features took 26 us in groups of 64 with
 // the mean at 20; a large list keeps long groups, which load their row once.

@@ -21,7 +21,7 @@ struct SpmmArgs {
   // values further
   long b_head_stride, c_head_stride, tc_vals_head_stride;
   int heads;  // grid.z of the ELL and tensor-core launches (0 or 1: one head)
-  int tc_slice_per;      // 128-feature slices per tensor-core CTA (blockIdx.y); set by the launcher
+  int tc_slice_per;      // 128-feature slices per tensor-core CTA (blockIdx.x); set by the launcher
   int tc_max_cta_steps;  // most k-steps the chunk schedule gives one CTA
   float* C;
   long ldc;

@@ -338,8 +338,9 @@ class DeviceSpmmPlan:
                    "stile_spmm_plan_set_wait_policy")
 
     def set_dvals_mode(self, mode: int):
-        """Value gradients of the tensor-tile nonzeros: 0 automatic, 1 on the
-        tensor cores, 2 by the row runs (stile_spmm_plan_set_dvals_mode)."""
+        """Value gradients of the tensor-tile nonzeros: 0 the default (the row
+        runs), 1 on the tensor cores, 2 by the row runs
+        (stile_spmm_plan_set_dvals_mode)."""
         _lib.check(self.lib.stile_spmm_plan_set_dvals_mode(self.handle, int(mode)), "stile_spmm_plan_set_dvals_mode")
 
     def error_flag(self) -> int:
